@@ -518,8 +518,9 @@ public:
             if (d[i] < 1 || d[i] > cap_) throw ArgError("checkpoint bond dimension exceeds this run's cap");
         for (int i = 0; i < n_; ++i) need += (size_t)d[i] * 2 * d[i + 1] * 16;
         if (bytes < need) throw ArgError("checkpoint truncated");
-        TQ_CK(cudaStreamSynchronize(stream_));
-        TQ_CK(cudaMemcpy(dims_, d.data(), sizeof(int) * (n_ + 1), cudaMemcpyHostToDevice));
+        // on the engine's own stream: a plain copy from pageable memory may still be in flight when
+        // it returns, and nothing would order it before the kernels of this non-blocking stream
+        TQ_CK(cudaMemcpyAsync(dims_, d.data(), sizeof(int) * (n_ + 1), cudaMemcpyHostToDevice, stream_));
         const char* q = p + ckpt_header_bytes(n_);
         std::vector<V> tmp;
         for (int i = 0; i < n_; ++i) {
@@ -532,11 +533,13 @@ public:
                 std::memcpy(&im, src + 2 * e + 1, 8);
                 tmp[e] = mk<V>((T)re, (T)im);
             }
-            TQ_CK(cudaMemcpy2D(sites_ + (size_t)i * site_stride(), cap_ * sizeof(V), tmp.data(), cols * sizeof(V),
-                               cols * sizeof(V), rows, cudaMemcpyHostToDevice));
+            TQ_CK(cudaMemcpy2DAsync(sites_ + (size_t)i * site_stride(), cap_ * sizeof(V), tmp.data(),
+                                    cols * sizeof(V), cols * sizeof(V), rows, cudaMemcpyHostToDevice, stream_));
+            TQ_CK(cudaStreamSynchronize(stream_));  // tmp is rewritten for the next site
             q += rows * cols * 16;
         }
-        TQ_CK(cudaMemset(stats_, 0, sizeof(RunStats)));
+        TQ_CK(cudaMemsetAsync(stats_, 0, sizeof(RunStats), stream_));
+        TQ_CK(cudaStreamSynchronize(stream_));
         ub_ = d;
     }
 
@@ -1016,15 +1019,17 @@ private:
         order_ = reinterpret_cast<int*>(base_ + a4);
         std::vector<InstTask<T>> it;
         for (int b = 0; b < B; ++b) it.push_back(eng_[b]->inst_task(step_, rows_cap_));
-        TQ_CK(cudaMemcpy(insts_, it.data(), sizeof(InstTask<T>) * B, cudaMemcpyHostToDevice));
-        if (nref_tot) TQ_CK(cudaMemcpy(refs_, refs.data(), sizeof(UpdRef) * nref_tot, cudaMemcpyHostToDevice));
+        TQ_CK(cudaMemcpyAsync(insts_, it.data(), sizeof(InstTask<T>) * B, cudaMemcpyHostToDevice, st_));
+        if (nref_tot) TQ_CK(cudaMemcpyAsync(refs_, refs.data(), sizeof(UpdRef) * nref_tot, cudaMemcpyHostToDevice, st_));
         if (!ops_all.empty())
-            TQ_CK(cudaMemcpy(ops_all_, ops_all.data(), sizeof(GateOp) * ops_all.size(), cudaMemcpyHostToDevice));
-        TQ_CK(cudaMemcpy(op_off_, op_off.data(), sizeof(int) * (B + 1), cudaMemcpyHostToDevice));
-        TQ_CK(cudaMemcpy(order_, order.data(), sizeof(int) * B, cudaMemcpyHostToDevice));
+            TQ_CK(cudaMemcpyAsync(ops_all_, ops_all.data(), sizeof(GateOp) * ops_all.size(), cudaMemcpyHostToDevice,
+                                  st_));
+        TQ_CK(cudaMemcpyAsync(op_off_, op_off.data(), sizeof(int) * (B + 1), cudaMemcpyHostToDevice, st_));
+        TQ_CK(cudaMemcpyAsync(order_, order.data(), sizeof(int) * B, cudaMemcpyHostToDevice, st_));
         resident_ = C[0].block == 0 && !C[0].theta_tc;
         theta_tc_ = C[0].theta_tc != 0;
         precond_ = C[0].precond != 2;
+        TQ_CK(cudaStreamSynchronize(st_));
         for (auto& e : eng_) TQ_CK(cudaStreamSynchronize(e->own_stream()));
     }
 

@@ -478,10 +478,13 @@ public:
         fill(Ly.Wg1, (size_t)H * H, H, 1.0);
         fill(Ly.Wg2, (size_t)(K - 1) * H, H, 0.1);
         set_params(hw.data());
-        GN_CK(cudaMemset(m1, 0, sizeof(float) * Ly.total * 2));
+        GN_CK(cudaMemsetAsync(m1, 0, sizeof(float) * Ly.total * 2, st));
     }
+    // Copies to the device go through `st`, the stream of the kernels that read them: a plain
+    // cudaMemcpy from pageable memory returns once the data is staged, and a kernel on this
+    // non-blocking stream could then read the weights before they have landed.
     void set_params(const float* host) {
-        GN_CK(cudaMemcpy(w, host, sizeof(float) * Ly.total, cudaMemcpyHostToDevice));
+        GN_CK(cudaMemcpyAsync(w, host, sizeof(float) * Ly.total, cudaMemcpyHostToDevice, st));
         k_to_bf16<<<grid_of(Ly.total), 256, 0, st>>>(w, Ly.total, wb);
         GN_CK(cudaGetLastError());
         GN_CK(cudaStreamSynchronize(st));
@@ -582,8 +585,7 @@ public:
     }
     // an externally reduced gradient (data-parallel training) into the gradient buffer
     void write_grads(const float* in) {
-        GN_CK(cudaStreamSynchronize(st));
-        GN_CK(cudaMemcpy(g, in, sizeof(float) * Ly.total, cudaMemcpyHostToDevice));
+        GN_CK(cudaMemcpyAsync(g, in, sizeof(float) * Ly.total, cudaMemcpyHostToDevice, st));
     }
     void read_grads(float* out) {
         GN_CK(cudaStreamSynchronize(st));
