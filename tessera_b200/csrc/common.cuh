@@ -134,6 +134,18 @@ __device__ __forceinline__ void tma_load_1d(void* dst, const void* src, unsigned
         "l"(src), "r"(bytes), "r"(smem_u32(bar))
         : "memory");
 }
+// shared -> global bulk copy (same alignment rules), completing by the issuing thread's bulk groups
+__device__ __forceinline__ void tma_store_1d(void* dst, const void* src, unsigned bytes) {
+    asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(dst), "r"(smem_u32(src)),
+                 "r"(bytes)
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+// this thread's bulk groups have read their shared-memory sources / are complete
+__device__ __forceinline__ void tma_store_wait_read() {
+    asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
+}
+__device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, unsigned parity) {
     unsigned ok;
     asm volatile(

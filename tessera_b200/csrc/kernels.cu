@@ -1944,6 +1944,558 @@ __device__ void svd_body_rc(const MpsView<T>& mps, const SvdWork<T>& wk, const S
                   red, flops);
 }
 
+// ------------------------------------------------------------------------------------
+// K2b in complex128: the same block-row-cyclic column-pair Jacobi with two resident columns per
+// warp, scaled rotations and tracked norms.
+//
+// One CTA per theta holds blocks of 2 NW columns in registers (warp w owns two columns, RPL rows
+// per lane) while the columns of the later blocks, NW at a time, stream past through two TMA
+// buffers.  A warp meets a streamed column y with both of its columns x1, x2 at once: one read of
+// y serves both inner products, which are reduced together, and one pass over y both rotations (y
+// stays in shared memory in between: its 64 registers would spill the columns).  The second
+// rotation needs x2^H y', y' being y after the first; with omega = x2^H x1 at hand that is
+// gamma2 + tau1 omega (up to scales), and omega itself follows from the same scalars.
+//
+//   * Norms: |x|^2 and |y|^2 are summed once per sweep and then follow from each rotation's
+//     c, tau and gamma, so a pair costs one inner product (4 multiply-adds per row) instead of
+//     three (12 operations).  A sweep starts from freshly summed norms, and convergence means a
+//     sweep without a rotation, so the last test is on summed norms and inner products only.
+//   * Scaled ("fast") rotations: the columns are kept as W = X diag(d) and a rotation is
+//     X1' = X1 - conj(tau) (d_y / d_1) Y, Y' = Y + tau (d_1 / d_y) X1 with d scaled by c: 8
+//     multiply-adds per row instead of 12.  d falls by at most 1/sqrt(2) per rotation and is
+//     folded back into the columns at the start of each sweep (at most 511 rotations later).
+//   * The angle tau is formed in FP32 from FP64 inputs scaled by a power of two; c = 1 / sqrt(1 +
+//     |tau|^2) is FP64, so the rotation is unitary to FP64 whatever tau is, and an angle good to
+//     1e-7 leaves 1e-7 of gamma, which the next sweep takes with the rest.
+//
+// Bound: the dots -> reduce -> angles -> update chain of a visit with two warps per scheduler (FP64
+// pipe 37 % busy: 12 multiply-adds per row and pair); shared memory moves 24 bytes per row and
+// pair.  148 graded 512 x 512 theta: 173 ms against 265 ms with one column per warp, three inner
+// products and unscaled rotations at the same 9.3 sweeps; 320 x 320: 65 against 94
+// ms.  Tried: y kept in registers
+// (183 ms, spills), no CTA barrier per J block but per-column hand-over (296 ms).
+// ------------------------------------------------------------------------------------
+constexpr int RCD_MAXN = 512;  // columns (2^-511 is the least a scale can reach within a sweep)
+
+__device__ __forceinline__ float sqrt_approx(const float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// 1 / sqrt(x) for x in [1, 4): an FP32 start y (relative error 1e-7) and one third-order step
+// y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2 of the series of (1 - e)^(-1/2), which leaves e^3
+__device__ __forceinline__ double rsqrt_near1(const double x) {
+    const double y = (double)rsqrtf((float)x);
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// tau = t e of the rotation w_p <- c (w_p - conj(tau) w_q), w_q <- c (w_q + tau w_p), from
+// alpha = |w_p|^2, beta = |w_q|^2, gamma = w_p^H w_q; false when the pair is converged or frozen.
+__device__ __forceinline__ bool jacobi_tau(const double a, const double b, const double gr, const double gi,
+                                           const double tol2, const double tiny, const bool mixed, double& tr,
+                                           double& ti) {
+    const double g2 = fma(gr, gr, gi * gi);
+    if (!(pair_live(a, b, tiny, mixed) && g2 > tol2 * (a * b))) return false;
+    // 2^-exponent(max(a, b)): the scaled values fit FP32 (|gamma| >= 1e-13 sqrt(a b) >= 1e-30 max)
+    const int e = (__double2hiint(fmax(a, b)) >> 20) & 0x7ff;
+    const double f = __hiloint2double((2046 - e) << 20, 0);
+    const float d = (float)((b - a) * f), xr = (float)(gr * f), xi = (float)(gi * f);
+    const float h = sqrt_approx(fmaf(d, d, 4.f * fmaf(xr, xr, xi * xi)));
+    const float s = __fdividef(d >= 0.f ? 2.f : -2.f, fabsf(d) + h);
+    tr = (double)(xr * s);
+    ti = (double)(xi * s);
+    return true;
+}
+
+// scale of a column (W = d X) and its reciprocal, after a rotation with cosine c: i = 1 / d kept to
+// rounding by one Newton step
+struct ColScale {
+    double d, i;
+    __device__ __forceinline__ void turn(const double c, const double t2) {
+        d *= c;
+        const double r = i * (c * (1.0 + t2));  // 1 / c = c (1 + t2)
+        i = r * fma(-d, r, 2.0);
+    }
+};
+
+// coefficients of a scaled rotation: X' = X - conj(tau) (d_y / d_x) Y, Y' = Y + tau (d_x / d_y) X
+struct RotCoef {
+    double br = 0.0, bi = 0.0, er = 0.0, ei = 0.0;  // none: the identity
+    __device__ __forceinline__ RotCoef() {}
+    __device__ __forceinline__ RotCoef(const double tr, const double ti, const ColScale& sx, const ColScale& sy) {
+        const double u = sx.d * sy.i, v = sy.d * sx.i;
+        br = -tr * v;
+        bi = ti * v;
+        er = tr * u;
+        ei = ti * u;
+    }
+    __device__ __forceinline__ void apply(double2& x, double2& y, const double2 xo, const double2 yo) const {
+        x.x = fma(-bi, yo.y, fma(br, yo.x, xo.x));
+        x.y = fma(bi, yo.x, fma(br, yo.y, xo.y));
+        y.x = fma(-ei, xo.y, fma(er, xo.x, yo.x));
+        y.y = fma(ei, xo.x, fma(er, xo.y, yo.y));
+    }
+};
+
+template <int RPL>
+__device__ __forceinline__ void lane_dot(const double2 (&x)[RPL], const double2 (&y)[RPL], double& re, double& im) {
+    double r0 = 0.0, r1 = 0.0, i0 = 0.0, i1 = 0.0;  // four chains
+#pragma unroll
+    for (int k = 0; k < RPL; ++k) {
+        r0 = fma(x[k].x, y[k].x, r0);
+        r1 = fma(x[k].y, y[k].y, r1);
+        i0 = fma(x[k].x, y[k].y, i0);
+        i1 = fma(-x[k].y, y[k].x, i1);
+    }
+    re = r0 + r1;
+    im = i0 + i1;
+}
+
+// sums of four doubles over the warp, to every lane: lanes hand over what they do not keep (two
+// values, then one), three levels on the one kept, and four broadcasts: 10 shuffles, not 20
+__device__ __forceinline__ void warp_sum4(double& a, double& b, double& c, double& d) {
+    const int lane = threadIdx.x & 31;
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const double s0 = __shfl_xor_sync(0xffffffffu, h16 ? a : c, 16);
+    const double s1 = __shfl_xor_sync(0xffffffffu, h16 ? b : d, 16);
+    const double p = (h16 ? c : a) + s0, q = (h16 ? d : b) + s1;
+    double v = (h8 ? q : p) + __shfl_xor_sync(0xffffffffu, h8 ? p : q, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    a = __shfl_sync(0xffffffffu, v, 0);
+    b = __shfl_sync(0xffffffffu, v, 8);
+    c = __shfl_sync(0xffffffffu, v, 16);
+    d = __shfl_sync(0xffffffffu, v, 24);
+}
+
+__device__ __forceinline__ void warp_sum2(double& a, double& b) {
+    const int lane = threadIdx.x & 31;
+    const bool h16 = lane & 16;
+    double v = (h16 ? b : a) + __shfl_xor_sync(0xffffffffu, h16 ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    a = __shfl_sync(0xffffffffu, v, 0);
+    b = __shfl_sync(0xffffffffu, v, 16);
+}
+
+template <int NW, int RPL>
+__device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& wk, const SvdParams& pp,
+                             unsigned char* smraw) {
+    constexpr int NT = 32 * NW, IB = 2 * NW, JB = NW;
+    __shared__ double red[4 * NW];
+    __shared__ int s_rot, s_ok, s_irot, s_jrot, s_fail;
+    __shared__ __align__(8) uint64_t bars[3];  // [0] block I, [1], [2] the two J buffers
+    __shared__ unsigned char cprev[RCD_MAXN], ccur[RCD_MAXN];  // columns changed last sweep / this one
+    __shared__ int perm[RCD_MAXN];                             // this sweep's order: descending norm
+    __shared__ double nrm[RCD_MAXN];                           // |w|^2 by column
+    __shared__ ColScale scl[RCD_MAXN];
+    __shared__ int s_ver[JB];  // rounds each J slot has been through since the SVD began
+    __shared__ double s_ws[NW][8];
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int R = pp.R > 0 ? pp.R : 2 * mps.dims[pp.bond];
+    const int N0 = pp.N > 0 ? pp.N : 2 * mps.dims[pp.bond + 2];
+    const int N = pp.lq && N0 > R ? R : N0;
+    constexpr int rc = 32 * RPL;  // staged column length; the rows from R on stay zero
+    const int ld = wk.ld;
+    double2* W = wk.W;
+    int* status = &wk.stats->status;
+    if (R > rc || N > RCD_MAXN) {  // host sizing bug guard
+        if (tid == 0) atomicOr(status, ST_BAD_DIMS);
+        return;
+    }
+    double2* buf = reinterpret_cast<double2*>(smraw);  // [2 JB][rc]: block I, then the two J buffers
+    if (tid == 0) {
+        for (int k = 0; k < 3; ++k) mbar_init(&bars[k], 1);
+        s_fail = 0;
+        s_jrot = 0;
+    }
+    if (tid < JB) s_ver[tid] = 0;
+    auto clear_tail = [&]() {  // (the sort keys of a sweep overlay the buffers)
+        for (int e = tid; e < IB * (rc - R); e += NT) buf[(e / (rc - R)) * rc + R + e % (rc - R)] = make_double2(0.0, 0.0);
+    };
+    for (int e = tid; e < N; e += NT) {
+        cprev[e] = 1;
+        ccur[e] = 1;
+        scl[e] = ColScale{1.0, 1.0};
+    }
+    __syncthreads();
+    unsigned ph[3] = {0u, 0u, 0u};
+    auto wait = [&](int k) -> bool {  // one CTA-wide outcome per copy wait
+        if (tid == 0) s_ok = mbar_wait(&bars[k], ph[k], 1000000000ull) ? 1 : 0;
+        __syncthreads();
+        const bool ok = s_ok != 0;
+        if (ok && tid != 0) mbar_wait(&bars[k], ph[k], 1000000000ull);
+        if (ok) ph[k] ^= 1u;
+        return ok;
+    };
+    // stage columns perm[p0 .. p0 + cnt) into dst (thread 0)
+    auto stage = [&](double2* dst, int p0, int cnt, uint64_t* bar) {
+        const int nv = N - p0 < cnt ? N - p0 : cnt;
+        const unsigned bytes = (unsigned)(R * sizeof(double2));
+        fence_proxy_async_shared();
+        mbar_expect_tx(bar, nv * bytes);
+        for (int c = 0; c < nv; ++c) tma_load_1d(dst + c * rc, W + (long long)perm[p0 + c] * ld, bytes, bar);
+    };
+    // exact norms of the columns changed since the last time, their scales folded into them
+    auto fold = [&](bool all) {
+        for (int j = warp; j < N; j += NW) {
+            if (!all && !ccur[j]) continue;
+            double2* w = W + (long long)j * ld;
+            const double d = scl[j].d;
+            double sj = 0.0;
+            for (int row = lane; row < R; row += 32) {
+                double2 v = w[row];
+                if (d != 1.0) {
+                    v.x *= d;
+                    v.y *= d;
+                    w[row] = v;
+                }
+                sj = fma(v.x, v.x, fma(v.y, v.y, sj));
+            }
+            sj = warp_sum(sj);
+            if (lane == 0) {
+                nrm[j] = sj;
+                scl[j] = ColScale{1.0, 1.0};
+            }
+        }
+        fence_proxy_async_global();  // bulk copies read these columns next
+        __syncthreads();
+    };
+    fold(true);
+    double fro2 = 0.0;
+    {
+        double part = 0.0;
+        for (int e = tid; e < N; e += NT) part += nrm[e];
+        part = warp_sum(part);
+        if (lane == 0) red[warp] = part;
+        __syncthreads();
+        for (int w = 0; w < NW; ++w) fro2 += red[w];
+    }
+    const double tiny = noise_tiny(pp.tiny, R, fro2, false);
+    const double tol2 = pp.tol * pp.tol;
+    __syncthreads();
+    const int nbi = (N + IB - 1) / IB, nbj = (N + JB - 1) / JB;
+    int vbase = 0;
+    double rots_total = 0.0, pairs_checked = 0.0;
+    double moved = (double)N;  // columns read or written (counted by thread 0)
+    auto dirty = [&](int p0, int cnt) {
+        bool d = false;
+        for (int p = p0; p < p0 + cnt && p < N; ++p) d = d || cprev[perm[p]] || ccur[perm[p]];
+        return d;
+    };
+    auto next_needed = [&](int j0, bool iflag) {  // first J block >= j0 whose pair with I needs a check
+        int j = j0;
+        while (j < nbj && !(iflag || dirty(j * JB, JB))) ++j;
+        return j;
+    };
+    int P2 = 1;
+    while (P2 < N) P2 <<= 1;
+    int sweep = 0;
+    bool converged = false, fail = false, mixed = true;
+    for (; sweep < pp.max_sweeps && !fail; ++sweep) {
+        if (sweep) {
+            fold(false);
+            moved += N;
+        }
+        if (tid == 0) s_rot = 0;
+        {   // descending norm order for this sweep; the staging buffer holds the sort keys
+            double* key = reinterpret_cast<double*>(smraw);
+            int* idx = reinterpret_cast<int*>(key + P2);
+            for (int c = tid; c < P2; c += NT) {
+                key[c] = c < N ? nrm[c] : -1.0;
+                idx[c] = c;
+            }
+            __syncthreads();
+            bitonic_desc(key, idx, P2);
+            for (int e = tid; e < N; e += NT) {
+                perm[e] = idx[e];
+                cprev[e] = ccur[e];
+                ccur[e] = 0;
+            }
+            __syncthreads();
+            if (R < rc) clear_tail();
+        }
+        int rot = 0;
+        for (int I = 0; I < nbi && !fail; ++I) {
+            const bool iflag = dirty(I * IB, IB);
+            int jn = next_needed((I + 1) * 2, iflag);
+            if (!iflag && jn >= nbj) continue;  // every pair of block I is unchanged and orthogonal
+            if (tid == 0) {
+                s_irot = 0;
+                stage(buf, I * IB, IB, &bars[0]);
+            }
+            moved += IB;
+            if (!wait(0)) { fail = true; break; }
+            if (iflag) {  // pairs inside block I: circle method, one warp per pair
+                pairs_checked += 0.5 * IB * (IB - 1);
+                for (int t = 0; t < IB - 1; ++t) {
+                    int p, q;
+                    tournament(IB, t, warp, p, q);
+                    if (I * IB + p < N && I * IB + q < N) {
+                        const int cp = perm[I * IB + p], cq = perm[I * IB + q];
+                        double2 x[RPL], y[RPL];
+#pragma unroll
+                        for (int k = 0; k < RPL; ++k) {
+                            const int row = lane + 32 * k;
+                            x[k] = buf[p * rc + row];
+                            y[k] = buf[q * rc + row];
+                        }
+                        double gr, gi, tr, ti;
+                        lane_dot<RPL>(x, y, gr, gi);
+                        warp_sum2(gr, gi);
+                        ColScale sx = scl[cp], sy = scl[cq];
+                        const double a = nrm[cp], b = nrm[cq], dd = sx.d * sy.d;
+                        gr *= dd;
+                        gi *= dd;
+                        if (jacobi_tau(a, b, gr, gi, tol2, tiny, mixed, tr, ti)) {
+                            const RotCoef rt(tr, ti, sx, sy);
+#pragma unroll
+                            for (int k = 0; k < RPL; ++k) {
+                                const int row = lane + 32 * k;
+                                const double2 xo = x[k], yo = y[k];
+                                rt.apply(x[k], y[k], xo, yo);
+                                buf[p * rc + row] = x[k];
+                                buf[q * rc + row] = y[k];
+                            }
+                            if (lane == 0) {
+                                const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2), g = fma(tr, gr, ti * gi);
+                                nrm[cp] = fmax(0.0, c * c * fma(t2, b, fma(-2.0, g, a)));
+                                nrm[cq] = fmax(0.0, c * c * fma(t2, a, fma(2.0, g, b)));
+                                sx.turn(c, t2);
+                                sy.turn(c, t2);
+                                scl[cp] = sx;
+                                scl[cq] = sy;
+                                ++rot;
+                                s_irot = 1;
+                            }
+                        }
+                    }
+                    __syncthreads();
+                }
+            }
+            // block I into registers: warp w takes columns 2w and 2w + 1
+            const int p1 = I * IB + 2 * warp, p2 = p1 + 1;
+            const int c1 = p1 < N ? perm[p1] : -1, c2 = p2 < N ? perm[p2] : -1;
+            double2 x1[RPL], x2[RPL];
+#pragma unroll
+            for (int k = 0; k < RPL; ++k) {
+                const int row = lane + 32 * k;
+                x1[k] = c1 >= 0 ? buf[(2 * warp) * rc + row] : make_double2(0.0, 0.0);
+                x2[k] = c2 >= 0 ? buf[(2 * warp + 1) * rc + row] : make_double2(0.0, 0.0);
+            }
+            // the two columns' norms, scales and omega = w_2^H w_1 live in shared memory: the rows take
+            // the registers
+            volatile double* ws = s_ws[warp];
+            {
+                const double a1 = c1 >= 0 ? nrm[c1] : 0.0, a2 = c2 >= 0 ? nrm[c2] : 0.0;
+                const ColScale s1 = c1 >= 0 ? scl[c1] : ColScale{1.0, 1.0};
+                const ColScale s2 = c2 >= 0 ? scl[c2] : ColScale{1.0, 1.0};
+                double wr, wi;
+                lane_dot<RPL>(x2, x1, wr, wi);
+                warp_sum2(wr, wi);
+                if (lane == 0) {
+                    ws[0] = a1; ws[1] = s1.d; ws[2] = s1.i;
+                    ws[3] = a2; ws[4] = s2.d; ws[5] = s2.i;
+                    ws[6] = wr * (s1.d * s2.d);
+                    ws[7] = wi * (s1.d * s2.d);
+                }
+            }
+            __syncthreads();  // buf free for the J blocks
+            if (jn < nbj && tid == 0) stage(buf, jn * JB, JB, &bars[1]);
+            int b = 0;
+            for (int J = jn; J < nbj; J = jn, b ^= 1) {
+                jn = next_needed(J + 1, iflag);
+                if (jn < nbj && tid == 0) {
+                    tma_store_wait_read();  // the copies out of that buffer have read it
+                    stage(buf + (b ^ 1) * JB * rc, jn * JB, JB, &bars[1 + (b ^ 1)]);
+                }
+                if (!wait(1 + b)) { fail = true; break; }
+                pairs_checked += (double)IB * JB;
+                moved += JB;
+                double2* cb = buf + b * JB * rc;
+                for (int t = 0; t < JB; ++t) {
+                    const int q = (warp + t) % JB;
+                    const bool ok = J * JB + q < N;
+                    const int cy = ok ? perm[J * JB + q] : 0;
+                    double2* cq = cb + q * rc + lane;
+                    if (t > 0) {  // bounded wait for warp w + 1 to release column q from round t - 1
+                        if (lane == 0) {
+                            const volatile int* vq = &s_ver[q];
+                            unsigned spin = 0;
+                            while (*vq < vbase + t && !*(volatile int*)&s_fail)
+                                if (++spin > (1u << 24)) { s_fail = 1; break; }
+                        }
+                        __syncwarp();
+                        __threadfence_block();
+                    }
+                    double g1r, g1i, g2r, g2i;
+                    {
+                        double u0 = 0, u1 = 0, u2 = 0, u3 = 0, v0 = 0, v1 = 0, v2 = 0, v3 = 0;
+#pragma unroll
+                        for (int k = 0; k < RPL; ++k) {
+                            const double2 y = cq[32 * k];
+                            u0 = fma(x1[k].x, y.x, u0);
+                            u1 = fma(x1[k].y, y.y, u1);
+                            u2 = fma(x1[k].x, y.y, u2);
+                            u3 = fma(-x1[k].y, y.x, u3);
+                            v0 = fma(x2[k].x, y.x, v0);
+                            v1 = fma(x2[k].y, y.y, v1);
+                            v2 = fma(x2[k].x, y.y, v2);
+                            v3 = fma(-x2[k].y, y.x, v3);
+                        }
+                        g1r = u0 + u1;
+                        g1i = u2 + u3;
+                        g2r = v0 + v1;
+                        g2i = v2 + v3;
+                    }
+                    double ay = ok ? *(volatile double*)&nrm[cy] : 0.0;
+                    ColScale sy{*(volatile double*)&scl[cy].d, *(volatile double*)&scl[cy].i};
+                    double a1 = ws[0], a2 = ws[3], wr = ws[6], wi = ws[7];
+                    ColScale s1{ws[1], ws[2]}, s2{ws[4], ws[5]};
+                    warp_sum4(g1r, g1i, g2r, g2i);
+                    const double d1 = s1.d * sy.d, d2 = s2.d * sy.d;
+                    g1r *= d1;
+                    g1i *= d1;
+                    g2r *= d2;
+                    g2i *= d2;
+                    // both angles first, then one pass over the rows for both rotations
+                    RotCoef q1, q2;
+                    double tr, ti, cc1 = 1.0, tt1 = 0.0;
+                    const bool t1 = jacobi_tau(a1, ay, g1r, g1i, tol2, tiny, mixed, tr, ti);
+                    if (t1) {
+                        const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2);
+                        const double g = fma(tr, g1r, ti * g1i), c2 = c * c;
+                        q1 = RotCoef(tr, ti, s1, sy);
+                        const double an = fmax(0.0, c2 * fma(t2, ay, fma(-2.0, g, a1)));
+                        ay = fmax(0.0, c2 * fma(t2, a1, fma(2.0, g, ay)));
+                        a1 = an;
+                        sy.turn(c, t2);
+                        // gamma2 = c (gamma2 + tau omega), omega = c (omega - conj(tau) gamma2)
+                        const double nr = c * fma(-ti, wi, fma(tr, wr, g2r));
+                        const double ni = c * fma(ti, wr, fma(tr, wi, g2i));
+                        wr = c * fma(-ti, g2i, fma(-tr, g2r, wr));
+                        wi = c * fma(ti, g2r, fma(-tr, g2i, wi));
+                        g2r = nr;
+                        g2i = ni;
+                        cc1 = c;
+                        tt1 = t2;
+                        if (lane == 0) ++rot;
+                    }
+                    const bool t2nd = jacobi_tau(a2, ay, g2r, g2i, tol2, tiny, mixed, tr, ti);
+                    if (t2nd) q2 = RotCoef(tr, ti, s2, sy);
+                    if (t1 || t2nd) {
+#pragma unroll
+                        for (int k = 0; k < RPL; ++k) {
+                            double2 v = cq[32 * k];
+                            const double2 xo = x1[k], zo = x2[k];
+                            q1.apply(x1[k], v, xo, v);
+                            q2.apply(x2[k], v, zo, v);
+                            cq[32 * k] = v;
+                        }
+                        if (t1) s1.turn(cc1, tt1);
+                        if (t2nd) {
+                            const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2);
+                            const double g = fma(tr, g2r, ti * g2i), c2 = c * c;
+                            const double an = fmax(0.0, c2 * fma(t2, ay, fma(-2.0, g, a2)));
+                            ay = fmax(0.0, c2 * fma(t2, a2, fma(2.0, g, ay)));
+                            a2 = an;
+                            s2.turn(c, t2);
+                            sy.turn(c, t2);
+                            wr *= c;  // x1^H y' was just annihilated
+                            wi *= c;
+                            if (lane == 0) ++rot;
+                        }
+                        if (lane == 0) {
+                            *(volatile double*)&nrm[cy] = ay;
+                            *(volatile double*)&scl[cy].d = sy.d;
+                            *(volatile double*)&scl[cy].i = sy.i;
+                            ws[0] = a1; ws[1] = s1.d; ws[2] = s1.i;
+                            ws[3] = a2; ws[4] = s2.d; ws[5] = s2.i;
+                            ws[6] = wr; ws[7] = wi;
+                            ccur[cy] = 1;
+                            s_jrot = 1;
+                            s_irot = 1;
+                        }
+                    }
+                    // release column q to warp w - 1 for round t + 1; the last round's columns go to
+                    // the bulk copies that write them back
+                    if (t == JB - 1) fence_proxy_async_shared();
+                    __syncwarp();
+                    __threadfence_block();
+                    if (lane == 0) *(volatile int*)&s_ver[q] = vbase + t + 1;
+                }
+                vbase += JB;
+                __syncthreads();
+                if (s_fail) { fail = true; break; }
+                if (tid == 0 && s_jrot) {  // block J back to global memory, asynchronously
+                    s_jrot = 0;  // set again only after the barrier of the next wait
+                    moved += JB;
+                    for (int c = 0; c < JB && J * JB + c < N; ++c)
+                        tma_store_1d(W + (long long)perm[J * JB + c] * ld, cb + c * rc, (unsigned)(R * sizeof(double2)));
+                    tma_store_commit();
+                }
+            }
+            if (tid == 0) tma_store_wait_all();  // block I + 1 and its J blocks read these columns
+            if (fail) break;
+            if (s_irot) {
+                moved += IB;
+                if (c1 >= 0) {
+                    double2* dst = W + (long long)c1 * ld;
+#pragma unroll
+                    for (int k = 0; k < RPL; ++k) {
+                        const int row = lane + 32 * k;
+                        if (row < R) dst[row] = x1[k];
+                    }
+                }
+                if (c2 >= 0) {
+                    double2* dst = W + (long long)c2 * ld;
+#pragma unroll
+                    for (int k = 0; k < RPL; ++k) {
+                        const int row = lane + 32 * k;
+                        if (row < R) dst[row] = x2[k];
+                    }
+                }
+                if (lane == 0) {
+                    if (c1 >= 0) { nrm[c1] = ws[0]; scl[c1] = ColScale{ws[1], ws[2]}; ccur[c1] = 1; }
+                    if (c2 >= 0) { nrm[c2] = ws[3]; scl[c2] = ColScale{ws[4], ws[5]}; ccur[c2] = 1; }
+                }
+            }
+            fence_proxy_async_global();
+            __syncthreads();
+        }
+        if (fail) break;
+        if (rot) atomicAdd(&s_rot, rot);
+        __syncthreads();
+        const int done = s_rot;
+        __syncthreads();
+        rots_total += done;
+        if (done == 0) {
+            converged = true;
+            ++sweep;
+            break;
+        }
+        mixed = still_mixed(mixed, done, N, sweep);
+    }
+    if (fail) {  // every thread leaves together; wait (bounded) for copies still in flight
+        if (tid == 0) {
+            atomicOr(status, ST_BARRIER_TIMEOUT);
+            for (int k = 0; k < 3; ++k) mbar_wait(&bars[k], ph[k], 1000000000ull);
+        }
+        __syncthreads();
+        return;
+    }
+    fold(true);  // the sweep cap may leave scales behind
+    for (int e = tid; e < N; e += NT) wk.sig2[e] = nrm[e];
+    __syncthreads();
+    moved += N;
+    // 8 flops per row of a pair checked (one complex inner product), 16 per row rotated
+    const double flops = pairs_checked * R * 8.0 + rots_total * R * 16.0;
+    svd_finish<double>(mps, wk, pp, R, N, fmax(1e-28, tiny), sweep, converged, moved * (double)R * sizeof(double2),
+                       smraw, red, flops);
+}
+
 // Batched: each CTA takes whole SVD tasks (one theta each) in turn; no inter-CTA waits.
 // lq: W holds the pivoted LQ factor P L of theta (lq.cu), whose columns beyond min(R, N) are zero.
 template <typename T, int BW, int RPL>
@@ -1956,8 +2508,8 @@ __global__ void __launch_bounds__(SvdShape<BW, RPL>::NT, 1) k_svd_batch(const In
         SvdParams pp = it.pp;
         pp.bond = rf.op.bond;
         pp.lq = lq;
-        if constexpr (RPL > 0) svd_body_rc<T, BW, RPL>(it.mps, it.wk, pp, smraw);
-        else svd_body<T, BW, RPL>(it.mps, it.wk, pp, 0, 1, smraw);
+        if constexpr (sizeof(T) == 8) svd_body_rcd<BW, RPL>(it.mps, it.wk, pp, smraw);
+        else svd_body_rc<T, BW, RPL>(it.mps, it.wk, pp, smraw);
         __syncthreads();
     }
 }
@@ -2518,8 +3070,8 @@ static void svd_batch_bw(const InstTask<T>* insts, const UpdRef* refs, int nref,
                          int lq = 0) {
     using V = cplx_t<T>;
     constexpr int NT = SvdShape<BW, RPL>::NT;
-    // block-row-cyclic (RPL > 0): block I plus two J buffers; else one staged block pair
-    size_t smem = sizeof(V) * (RPL > 0 ? 3 : 2) * BW * (size_t)rows_cap;
+    // complex64: block I plus two J buffers; complex128: two J buffers, which also stage block I
+    size_t smem = sizeof(V) * (sizeof(T) == 8 ? 2 * BW * 32 * RPL : 3 * BW * (size_t)rows_cap);
     const size_t sort_smem = 4096 * (sizeof(double) + sizeof(int));
     if (smem < sort_smem) smem = sort_smem;
     auto fn = k_svd_batch<T, BW, RPL>;
@@ -2533,14 +3085,16 @@ static void svd_batch_bw(const InstTask<T>* insts, const UpdRef* refs, int nref,
     TQ_CHECK(cudaGetLastError());
 }
 
-// complex64 at 512 rows: blocks of 16 columns (512 threads, 16 warps); a complex128 column pair
-// of 512 rows does not fit in the registers that 16 warps leave each thread
-template <typename T>
-static bool svd_batch_wide(const InstTask<T>* insts, const UpdRef* refs, int nref, int rows_cap, cudaStream_t s,
-                           int lq) {
+// complex64: blocks of 16 columns (512 threads, 16 warps); complex128 columns do not fit in the
+// registers that 16 warps leave each thread
+template <typename T, int RPL>
+static bool svd_batch_wide(int bw, int rpl, const InstTask<T>* insts, const UpdRef* refs, int nref, int rows_cap,
+                           cudaStream_t s, int lq) {
     if constexpr (sizeof(T) == 4) {
-        svd_batch_bw<T, 16, 16>(insts, refs, nref, rows_cap, s, lq);
-        return true;
+        if (bw == 16 && rpl == RPL) {
+            svd_batch_bw<T, 16, RPL>(insts, refs, nref, rows_cap, s, lq);
+            return true;
+        }
     }
     return false;
 }
@@ -2576,6 +3130,7 @@ int launch_update_batch(const InstTask<T>* insts, const UpdRef* refs, int nref, 
     // one asked for; complex64 at 257..512 rows: 16), or the block-Gram kernel when block width
     // 32 is asked for
     if (block_w == 0) bw = (sizeof(T) == 4 && rpl == 16) ? 16 : 8;
+    if (sizeof(T) == 8 && bw > 8) bw = 8;  // two columns a warp: 16 warps leave too few registers
     // the pivoted LQ preconditioner for the column-pair kernel at 257..512 rows (outside the
     // svd_begin/svd_end window, so that window times the Jacobi alone)
     const int lq = (precond && block_w != BG_B && rpl == 16 && resident_smem<T>(rows_cap, rows_cap) == 0) ? 1 : 0;
@@ -2589,14 +3144,14 @@ int launch_update_batch(const InstTask<T>* insts, const UpdRef* refs, int nref, 
     if (res_dispatch<T>(nullptr, nullptr, rp, insts, refs, nref, s)) {
     } else if (block_w == BG_B) {
         bgj_launch<T>(nullptr, nullptr, nullptr, insts, refs, nref, s);
-    } else if (bw == 16 && rpl == 16 && svd_batch_wide<T>(insts, refs, nref, rows_cap, s, lq)) {
+    } else if (svd_batch_wide<T, 16>(bw, rpl, insts, refs, nref, rows_cap, s, lq)) {
     } else {
 #define TQ_RB(B, RP) \
     if (bw == B && rpl == RP) { svd_batch_bw<T, B, RP>(insts, refs, nref, rows_cap, s, lq); } else
-        TQ_RB(4, 1) TQ_RB(4, 2) TQ_RB(4, 4) TQ_RB(4, 8) TQ_RB(4, 16)
-        TQ_RB(8, 1) TQ_RB(8, 2) TQ_RB(8, 4) TQ_RB(8, 8) TQ_RB(8, 16)
-        TQ_RB(16, 1) TQ_RB(16, 2) TQ_RB(16, 4) TQ_RB(16, 8)
-        throw std::runtime_error("unsupported Jacobi block width");
+        // (theta up to 64 rows is resident in either precision)
+        TQ_RB(4, 4) TQ_RB(4, 8) TQ_RB(4, 16) TQ_RB(8, 4) TQ_RB(8, 8) TQ_RB(8, 16)
+        if (!svd_batch_wide<T, 8>(bw, rpl, insts, refs, nref, rows_cap, s, lq))
+            throw std::runtime_error("unsupported Jacobi block width");
 #undef TQ_RB
     }
     if (svd_end) TQ_CHECK(cudaEventRecord(svd_end, s));
