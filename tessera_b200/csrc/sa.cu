@@ -10,9 +10,21 @@
 // splitmix64 stream keyed by (seed, instance, restart, sweep, spin), so a run is reproducible
 // and the CPU oracle restates it draw for draw.
 //
-// Layout: one CTA per instance, one thread per restart chain (chunks of SA_THREADS restarts).
-// The coupling graph sits in shared memory as adjacency lists (offsets, neighbour, weight);
-// a chain's spins are a bit mask of SA_MAXN bits in registers (bit i set <-> s_i = -1).
+// Layout: SA_G lanes per restart chain, as many CTAs per instance as it takes to fill the GPU (each
+// strides over the instance's restarts); the last CTA of an instance to finish picks the winner.
+// The coupling graph sits in shared memory as adjacency lists (offsets, neighbour, weight; repeated
+// pairs merged); a chain's spins are a bit mask of SA_MAXN bits in registers (bit i set <-> s_i =
+// -1), and its local fields h_i + sum_j J_ij s_j are kept in shared memory and changed only where a
+// flip changes them, the chain's lanes sharing the neighbours.  A visit that does not flip, the
+// usual one once the chain has cooled, costs no walk over the neighbours.  Each lane draws the
+// uniform of every SA_G-th spin and the temperature of every SA_G-th sweep, and shuffles hand them
+// round.  The Metropolis test is decided in FP32 where FP32 can tell, u outside (1 -+ 1e-4) exp(-dE
+// / t), and by the FP64 exp otherwise, so every decision is the FP64 one.
+//
+// Bound: the latency of a visit (shuffle, field, test, a flip's walk).  8 dense n = 48 instances,
+// 512 restarts x 500 sweeps: 84 ms with one thread per chain, 128 chains a CTA and the field summed
+// at every visit; 20.5 ms with one CTA per 32 chains and kept fields (a warp then walks at nearly
+// every visit, for whichever chain flips); 6.4 ms with 8 lanes per chain.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -29,7 +41,10 @@ namespace tq {
 
 constexpr int SA_MAXN = 128;
 constexpr int SA_WORDS = SA_MAXN / 64;
+constexpr int SA_G = 8;            // lanes per chain
 constexpr int SA_THREADS = 128;
+constexpr int SA_CHAINS = SA_THREADS / SA_G;  // 16: their fields (16 KB at 128 spins) fit beside any graph
+constexpr int SA_CTAS_PER_SM = 8;  // CTAs to aim at before a CTA takes more than one turn of restarts
 
 #define SA_CK(x)                                                                                          \
     do {                                                                                                  \
@@ -55,51 +70,91 @@ struct SaTask {
     int m;     // its edges (self-loops included: they enter the energy)
 };
 
+// best chain of one CTA
+struct SaBest {
+    double e;
+    int r;  // restart, -1 = none below infinity
+    int pad;
+    unsigned long long bits[SA_WORDS];
+};
+
+// lower energy first, then the lower restart; r < 0 never wins
+__device__ __forceinline__ bool sa_before(const double e, const int r, const double e2, const int r2) {
+    if (r < 0 || r2 < 0) return r >= 0;
+    return e < e2 || (e == e2 && r < r2);
+}
+
 __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const int* adj_off, const int* adj_nbr,
                                                    const double* adj_w, const double* h, const int* ei, const int* ej,
                                                    const double* ew, int restarts, int sweeps, double t0,
-                                                   double t_end, unsigned long long seed, double* out_e,
-                                                   int8_t* out_s) {
+                                                   double t_end, unsigned long long seed, SaBest* part, int* tickets,
+                                                   double* out_e, int8_t* out_s) {
     extern __shared__ __align__(16) unsigned char smraw[];
     const SaTask tk = tasks[blockIdx.x];
+    const int tid = threadIdx.x, chain = tid / SA_G, gl = tid % SA_G;
     const int n = tk.n, a0 = adj_off[tk.hoff], deg_tot = adj_off[tk.hoff + n] - a0;
-    double* sw = reinterpret_cast<double*>(smraw);     // [deg_tot] weights
-    double* sh = sw + deg_tot;                         // [n] fields
-    int* so = reinterpret_cast<int*>(sh + n);          // [n + 1] offsets
-    short* sn = reinterpret_cast<short*>(so + n + 1);  // [deg_tot] neighbours
-    __shared__ double s_best[SA_THREADS];
-    __shared__ int s_arg[SA_THREADS];
-    __shared__ unsigned long long s_bits[SA_THREADS][SA_WORDS];
-    for (int e = threadIdx.x; e < deg_tot; e += blockDim.x) {
+    double* fld = reinterpret_cast<double*>(smraw) + chain * n;      // [n] this chain's local fields
+    double* sw = reinterpret_cast<double*>(smraw) + SA_CHAINS * n;   // [deg_tot] weights
+    double* sh = sw + deg_tot;                                       // [n] fields
+    int* so = reinterpret_cast<int*>(sh + n);                        // [n + 1] offsets
+    short* sn = reinterpret_cast<short*>(so + n + 1);                // [deg_tot] neighbours
+    __shared__ SaBest s_best[SA_CHAINS];
+    __shared__ int s_last;
+    for (int e = tid; e < deg_tot; e += SA_THREADS) {
         sw[e] = adj_w[a0 + e];
         sn[e] = (short)adj_nbr[a0 + e];
     }
-    for (int i = threadIdx.x; i < n; i += blockDim.x) sh[i] = h[tk.hoff + i];
-    for (int i = threadIdx.x; i <= n; i += blockDim.x) so[i] = adj_off[tk.hoff + i] - a0;
+    for (int i = tid; i < n; i += SA_THREADS) sh[i] = h[tk.hoff + i];
+    for (int i = tid; i <= n; i += SA_THREADS) so[i] = adj_off[tk.hoff + i] - a0;
     __syncthreads();
     const double ratio = t_end / t0;
     const double den = (double)((sweeps < 2 ? 2 : sweeps) - 1);
-    double best = INFINITY;
-    int best_r = -1;
-    unsigned long long best_bits[SA_WORDS] = {};
-    for (int r0 = 0; r0 < restarts; r0 += blockDim.x) {
-        const int r = r0 + threadIdx.x;
-        if (r >= restarts) break;
+    SaBest best{INFINITY, -1, 0, {}};
+    // every lane of a warp takes the same turns (a chain past the last restart runs along unseen)
+    for (int r0 = blockIdx.y * SA_CHAINS; r0 < restarts; r0 += gridDim.y * SA_CHAINS) {
+        const int r = r0 + chain;
         unsigned long long bits[SA_WORDS] = {};
         for (int i = 0; i < n; ++i)  // random start: s_i = -1 with probability 1/2
             if (sa_uniform(seed, blockIdx.x, r, sweeps, i, sweeps, n) < 0.5) bits[i >> 6] |= 1ull << (i & 63);
+        for (int i = gl; i < n; i += SA_G) {
+            double f = sh[i];
+            for (int e = so[i]; e < so[i + 1]; ++e) {
+                const int j = sn[e];
+                f += ((bits[j >> 6] >> (j & 63)) & 1ull) ? -sw[e] : sw[e];
+            }
+            fld[i] = f;
+        }
+        __syncwarp();
+        double tl = 0.0;
         for (int k = 0; k < sweeps; ++k) {
-            const double t = t0 * pow(ratio, (double)k / den);
-            for (int i = 0; i < n; ++i) {
-                double f = sh[i];
-                for (int e = so[i]; e < so[i + 1]; ++e) {
-                    const int j = sn[e];
-                    f += ((bits[j >> 6] >> (j & 63)) & 1ull) ? -sw[e] : sw[e];
+            if (k % SA_G == 0) tl = t0 * pow(ratio, (double)(k + gl) / den);
+            const double t = __shfl_sync(0xffffffffu, tl, k % SA_G, SA_G);
+            const float it = (float)(1.0 / t);
+            for (int i0 = 0; i0 < n; i0 += SA_G) {
+                const double ul = sa_uniform(seed, blockIdx.x, r, k, i0 + gl, sweeps, n);
+                const int i1 = n - i0 < SA_G ? n - i0 : SA_G;
+                for (int s = 0; s < i1; ++s) {
+                    const int i = i0 + s;
+                    const double u = __shfl_sync(0xffffffffu, ul, s, SA_G);
+                    const bool neg = (bits[i >> 6] >> (i & 63)) & 1ull;
+                    const double f = fld[i];
+                    const double de = 2.0 * (neg ? -f : f);
+                    bool flip = de < 0.0;
+                    if (!flip) {
+                        const float p = __expf(-(float)de * it), v = (float)u;
+                        if (v < p * 0.9999f) flip = true;
+                        else if (!(v > p * 1.0001f) || v == 0.f) flip = u < exp(-de / t);  // FP32 cannot tell
+                    }
+                    if (flip) {
+                        bits[i >> 6] ^= 1ull << (i & 63);
+                        const int e1 = so[i + 1];
+                        for (int e = so[i] + gl; e < e1; e += SA_G) {  // s_i changed by +2 if it was -1, else -2
+                            const double w2 = 2.0 * sw[e];
+                            fld[sn[e]] += neg ? w2 : -w2;
+                        }
+                    }
+                    __syncwarp();
                 }
-                const bool neg = (bits[i >> 6] >> (i & 63)) & 1ull;
-                const double de = 2.0 * (neg ? -f : f);
-                if (de < 0.0 || sa_uniform(seed, blockIdx.x, r, k, i, sweeps, n) < exp(-de / t))
-                    bits[i >> 6] ^= 1ull << (i & 63);
             }
         }
         double en = 0.0;  // E = -sum w s_i s_j - sum h s_i, in the order of the edge list
@@ -109,25 +164,37 @@ __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const in
             en -= (si == sj) ? ew[tk.eoff + e] : -ew[tk.eoff + e];
         }
         for (int i = 0; i < n; ++i) en -= ((bits[i >> 6] >> (i & 63)) & 1ull) ? -sh[i] : sh[i];
-        if (en < best) {
-            best = en;
-            best_r = r;
-            for (int w = 0; w < SA_WORDS; ++w) best_bits[w] = bits[w];
+        if (r < restarts && en < best.e) {
+            best.e = en;
+            best.r = r;
+            for (int w = 0; w < SA_WORDS; ++w) best.bits[w] = bits[w];
         }
+        __syncwarp();
     }
-    s_best[threadIdx.x] = best;
-    s_arg[threadIdx.x] = best_r;
-    for (int w = 0; w < SA_WORDS; ++w) s_bits[threadIdx.x][w] = best_bits[w];
+    if (gl == 0) s_best[chain] = best;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (tid == 0) {
         int bt = 0;
-        for (int t = 1; t < (int)blockDim.x; ++t) {
-            if (s_arg[t] < 0) continue;
-            if (s_best[t] < s_best[bt] || (s_best[t] == s_best[bt] && s_arg[t] < s_arg[bt])) bt = t;
+        for (int t = 1; t < SA_CHAINS; ++t)
+            if (sa_before(s_best[t].e, s_best[t].r, s_best[bt].e, s_best[bt].r)) bt = t;
+        part[(size_t)blockIdx.x * gridDim.y + blockIdx.y] = s_best[bt];
+        __threadfence();
+        s_last = atomicAdd(&tickets[blockIdx.x], 1) == (int)gridDim.y - 1;
+        if (s_last) {  // the instance's last CTA: its winner over all CTAs
+            __threadfence();
+            const SaBest* p = part + (size_t)blockIdx.x * gridDim.y;
+            int bc = 0;
+            for (int c = 1; c < (int)gridDim.y; ++c)
+                if (sa_before(__ldcg(&p[c].e), __ldcg(&p[c].r), __ldcg(&p[bc].e), __ldcg(&p[bc].r))) bc = c;
+            s_best[0].e = __ldcg(&p[bc].e);
+            for (int w = 0; w < SA_WORDS; ++w) s_best[0].bits[w] = __ldcg(&p[bc].bits[w]);
+            out_e[blockIdx.x] = s_best[0].e;
         }
-        out_e[blockIdx.x] = s_best[bt];
-        for (int i = 0; i < n; ++i) out_s[tk.hoff + i] = ((s_bits[bt][i >> 6] >> (i & 63)) & 1ull) ? -1 : 1;
     }
+    __syncthreads();
+    if (s_last)
+        for (int i = tid; i < n; i += SA_THREADS)
+            out_s[tk.hoff + i] = ((s_best[0].bits[i >> 6] >> (i & 63)) & 1ull) ? -1 : 1;
 }
 
 void set_last_error(const std::string& msg);  // engine.cu: the message tessera_qa_last_error() returns
@@ -160,6 +227,7 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
         // given (self-loops included, as Ising::energy does); the dynamics skip self-loops,
         // which only add a constant.
         std::vector<SaTask> tasks(count);
+        std::vector<int> where;  // (spin, spin) -> its place in the first spin's list
         std::vector<int> adj_off, nbr, ei, ej;
         std::vector<double> w, h, ew;
         size_t smem = 0;
@@ -170,6 +238,8 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
                                             std::to_string(SA_MAXN) + " and non-NULL arrays");
             const int n = (int)p.n;
             std::vector<std::vector<std::pair<int, double>>> adj(n);
+            where.assign(p.n * p.n, -1);
+            size_t listed = 0;  // entries as given, repeated pairs and all: what the size limit counts
             for (int i = 0; i < n; ++i)
                 if (!std::isfinite(p.h[i])) throw std::invalid_argument("non-finite field");
             SaTask t{n, (int)h.size(), (int)ei.size(), (int)p.m};
@@ -181,10 +251,19 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
                 ej.push_back((int)j);
                 ew.push_back(p.ew[e]);
                 if (i == j) continue;
-                adj[i].push_back({(int)j, p.ew[e]});
-                adj[j].push_back({(int)i, p.ew[e]});
+                listed += 2;
+                for (int side = 0; side < 2; ++side) {  // a repeated pair adds to its first entry
+                    auto& row = adj[side ? j : i];
+                    const int other = (int)(side ? i : j);
+                    int& at = where[(side ? j : i) * p.n + other];
+                    if (at < 0) {
+                        at = (int)row.size();
+                        row.push_back({other, p.ew[e]});
+                    } else {
+                        row[at].second += p.ew[e];
+                    }
+                }
             }
-            size_t deg = 0;
             for (int i = 0; i < n; ++i) {
                 h.push_back(p.h[i]);
                 adj_off.push_back((int)nbr.size());
@@ -192,22 +271,31 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
                     nbr.push_back(pr.first);
                     w.push_back(pr.second);
                 }
-                deg += adj[i].size();
             }
             tasks[b] = t;
-            smem = std::max(smem, deg * (sizeof(double) + sizeof(short)) + n * sizeof(double) +
+            smem = std::max(smem, listed * (sizeof(double) + sizeof(short)) + n * sizeof(double) +
                                       (n + 1) * sizeof(int) + 64);
         }
         adj_off.push_back((int)nbr.size());
         if (smem > 200 * 1024) throw std::invalid_argument("instance graph too large for shared memory");
+        size_t nmax = 0;
+        for (const SaTask& t : tasks) nmax = std::max(nmax, (size_t)t.n);
+        smem += nmax * SA_CHAINS * sizeof(double);
+        int dev = 0, sms = 0;
+        SA_CK(cudaGetDevice(&dev));
+        SA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        // CTAs per instance: one turn of restarts each, unless the batch alone fills the GPU
+        const size_t turns = (restarts + SA_CHAINS - 1) / SA_CHAINS;
+        const size_t share = std::max<size_t>(1, ((size_t)sms * SA_CTAS_PER_SM + count - 1) / count);
+        const size_t ctas = std::min(turns, share);
         auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
         const size_t b_tasks = al(sizeof(SaTask) * count), b_off = al(sizeof(int) * adj_off.size()),
                      b_nbr = al(sizeof(int) * std::max<size_t>(nbr.size(), 1)),
                      b_w = al(sizeof(double) * std::max<size_t>(w.size(), 1)), b_h = al(sizeof(double) * h.size()),
                      b_ei = al(sizeof(int) * std::max<size_t>(ei.size(), 1)),
                      b_ew = al(sizeof(double) * std::max<size_t>(ew.size(), 1)), b_e = al(sizeof(double) * count),
-                     b_s = al(h.size());
-        const size_t total = b_tasks + b_off + b_nbr + b_w + b_h + 2 * b_ei + b_ew + b_e + b_s;
+                     b_s = al(h.size()), b_part = al(sizeof(SaBest) * count * ctas), b_tick = al(sizeof(int) * count);
+        const size_t total = b_tasks + b_off + b_nbr + b_w + b_h + 2 * b_ei + b_ew + b_e + b_s + b_part + b_tick;
         SA_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         SA_CK(device_alloc((void**)&arena, total));
         char* q = arena;
@@ -222,6 +310,9 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
         double* d_ew = (double*)take(b_ew);
         double* d_e = (double*)take(b_e);
         int8_t* d_s = (int8_t*)take(b_s);
+        SaBest* d_part = (SaBest*)take(b_part);
+        int* d_tick = (int*)take(b_tick);
+        SA_CK(cudaMemsetAsync(d_tick, 0, sizeof(int) * count, st));
         auto up = [&](void* d, const void* hsrc, size_t bytes) {
             if (bytes) SA_CK(cudaMemcpyAsync(d, hsrc, bytes, cudaMemcpyHostToDevice, st));
         };
@@ -234,9 +325,9 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
         up(d_ej, ej.data(), sizeof(int) * ej.size());
         up(d_ew, ew.data(), sizeof(double) * ew.size());
         SA_CK(cudaFuncSetAttribute(k_sa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        const int threads = (int)std::min<size_t>(restarts, SA_THREADS);
-        k_sa<<<(unsigned)count, threads, smem, st>>>(d_tasks, d_off, d_nbr, d_w, d_h, d_ei, d_ej, d_ew,
-                                                     (int)restarts, (int)sweeps, t0, t_end, seed, d_e, d_s);
+        k_sa<<<dim3((unsigned)count, (unsigned)ctas), SA_THREADS, smem, st>>>(d_tasks, d_off, d_nbr, d_w, d_h, d_ei, d_ej,
+                                                                          d_ew, (int)restarts, (int)sweeps, t0, t_end,
+                                                                          seed, d_part, d_tick, d_e, d_s);
         SA_CK(cudaGetLastError());
         std::vector<double> e(count);
         std::vector<int8_t> s(h.size());
