@@ -19,6 +19,7 @@
 #include <mutex>
 #include <stdexcept>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "../../include/tessera_qa.h"
@@ -49,6 +50,91 @@ static void set_err(const std::string& s) { t_err = s; }
 static std::mutex g_fail_mu;
 static int g_fail_after = 0, g_fail_count = 0;
 
+// The library's own memory pool on each device.  cudaMalloc and cudaFree map and unmap pages and
+// wait for the whole device: on one box 0.1 ms a pair, on another 3 ms, and more for 100 MB, beside
+// kernels of a few microseconds; a call that makes an engine, runs it and drops it paid that several
+// times.  Freed memory stays in the pool up to kKeep bytes per device; what is above goes back to
+// the driver at each free, all of it when an allocation fails or device_trim() is called, and the
+// pools end with the process.  Allocation and release run on a stream of the pool's own that no
+// kernel uses, and are waited for, so the memory is good for any stream and thread when alloc()
+// returns; callers have waited for their work before they free, as cudaFree's callers had not to.
+class DevicePools {
+public:
+    static DevicePools& get() {
+        static DevicePools* p = new DevicePools;  // never destroyed: engines may outlive static objects
+        return *p;
+    }
+    cudaError_t alloc(void** out, size_t bytes) {
+        int dev = 0;
+        cudaError_t e = cudaGetDevice(&dev);
+        if (e != cudaSuccess) return e;
+        std::lock_guard<std::mutex> lk(mu_);
+        Pool* pl = pool(dev);
+        if (!pl) return cudaMalloc(out, bytes);
+        for (int turn = 0; turn < 2; ++turn) {
+            e = cudaMallocFromPoolAsync(out, bytes, pl->pool, pl->st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(pl->st);
+            if (e != cudaErrorMemoryAllocation) break;
+            cudaGetLastError();  // not sticky: the caller reports it, or the second turn succeeds
+            if (turn == 0) cudaMemPoolTrimTo(pl->pool, 0);
+        }
+        if (e == cudaSuccess) owner_[*out] = dev;
+        return e;
+    }
+    void free(void* p) {
+        if (!p) return;
+        std::lock_guard<std::mutex> lk(mu_);
+        auto it = owner_.find(p);
+        if (it == owner_.end()) {
+            cudaFree(p);
+            return;
+        }
+        Pool& pl = pools_[it->second];
+        owner_.erase(it);
+        cudaFreeAsync(p, pl.st);
+        cudaStreamSynchronize(pl.st);
+    }
+    void trim() {
+        std::lock_guard<std::mutex> lk(mu_);
+        int dev = 0;
+        if (cudaGetDevice(&dev) == cudaSuccess && dev < kMax && pools_[dev].state == 1) cudaMemPoolTrimTo(pools_[dev].pool, 0);
+    }
+
+private:
+    static constexpr int kMax = 64;
+    static constexpr uint64_t kKeep = 256ull << 20;
+    struct Pool {
+        int state = 0;  // 0 not tried, 1 ready, 2 not to be had on this device
+        cudaMemPool_t pool = nullptr;
+        cudaStream_t st = nullptr;
+    };
+    Pool* pool(int dev) {  // dev is current; nullptr: plain cudaMalloc
+        if (dev < 0 || dev >= kMax) return nullptr;
+        Pool& pl = pools_[dev];
+        if (pl.state == 0) {
+            pl.state = 2;
+            int ok = 0;
+            cudaMemPoolProps pr;
+            std::memset(&pr, 0, sizeof(pr));
+            pr.allocType = cudaMemAllocationTypePinned;
+            pr.location.type = cudaMemLocationTypeDevice;
+            pr.location.id = dev;
+            uint64_t keep = kKeep;
+            if (cudaDeviceGetAttribute(&ok, cudaDevAttrMemoryPoolsSupported, dev) == cudaSuccess && ok &&
+                cudaStreamCreateWithFlags(&pl.st, cudaStreamNonBlocking) == cudaSuccess &&
+                cudaMemPoolCreate(&pl.pool, &pr) == cudaSuccess &&
+                cudaMemPoolSetAttribute(pl.pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+                pl.state = 1;
+            else
+                cudaGetLastError();
+        }
+        return pl.state == 1 ? &pl : nullptr;
+    }
+    std::mutex mu_;
+    Pool pools_[kMax];
+    std::unordered_map<void*, int> owner_;
+};
+
 cudaError_t device_alloc(void** p, size_t bytes) {
     {
         std::lock_guard<std::mutex> lk(g_fail_mu);
@@ -62,8 +148,10 @@ cudaError_t device_alloc(void** p, size_t bytes) {
             }
         }
     }
-    return cudaMalloc(p, bytes);
+    return DevicePools::get().alloc(p, bytes);
 }
+void device_free(void* p) { DevicePools::get().free(p); }
+void device_trim() { DevicePools::get().trim(); }
 void set_last_error(const std::string& msg) { t_err = msg; }
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
@@ -249,9 +337,9 @@ public:
         for (cudaEvent_t e : pool_) cudaEventDestroy(e);
         if (ev0_) cudaEventDestroy(ev0_);
         if (ev1_) cudaEventDestroy(ev1_);
-        if (base_) cudaFree(base_);
-        if (res_base_) cudaFree(res_base_);
-        if (obs_) cudaFree(obs_);
+        if (base_) device_free(base_);
+        if (res_base_) device_free(res_base_);
+        if (obs_) device_free(obs_);
         if (stream_) cudaStreamDestroy(stream_);
         pool_.clear();
         ev0_ = ev1_ = nullptr;
@@ -454,12 +542,12 @@ public:
         try {
             launch_sample<T>(M, obs_, (int)count, seed, d, stream_);
         } catch (...) {
-            cudaFree(d);
+            device_free(d);
             throw;
         }
         err = cudaMemcpyAsync(spins, d, count * (size_t)n_, cudaMemcpyDeviceToHost, stream_);
         if (err == cudaSuccess) err = cudaStreamSynchronize(stream_);
-        cudaFree(d);
+        device_free(d);
         TQ_CK(err);
         if (energies)
             for (size_t c = 0; c < count; ++c) {
@@ -953,7 +1041,7 @@ public:
         for (cudaEvent_t e : pool_) cudaEventDestroy(e);
         if (e0_) cudaEventDestroy(e0_);
         if (e1_) cudaEventDestroy(e1_);
-        if (base_) cudaFree(base_);
+        if (base_) device_free(base_);
         if (st_) cudaStreamDestroy(st_);
         pool_.clear();
         e0_ = e1_ = nullptr;

@@ -35,7 +35,8 @@
 
 namespace tq {
 
-cudaError_t device_alloc(void** p, size_t bytes);  // engine.cu: cudaMalloc with failure injection
+cudaError_t device_alloc(void** p, size_t bytes);  // engine.cu: the library's pool, with failure injection
+void device_free(void* p);
 
 void set_last_error(const std::string& msg);
 
@@ -437,9 +438,9 @@ public:
     ~Gnn() { release(); }
     void release() noexcept {
         if (st) cudaStreamSynchronize(st);
-        if (arena) cudaFree(arena);
-        if (w) cudaFree(w);
-        if (wb) cudaFree(wb);
+        if (arena) device_free(arena);
+        if (w) device_free(w);
+        if (wb) device_free(wb);
         if (st) cudaStreamDestroy(st);
         arena = nullptr;
         w = nullptr;
@@ -612,7 +613,7 @@ private:
         if (nG <= capG && nN <= capN && nE <= capE) return;
         if (arena) {
             GN_CK(cudaStreamSynchronize(st));
-            cudaFree(arena);
+            device_free(arena);
         }
         arena = nullptr;
         capG = std::max(nG, 1);
@@ -767,7 +768,7 @@ double tessera_qa_exact_ground(const double* h, size_t n, const size_t* ei, cons
         std::vector<unsigned long long> hx(blocks);
         if (err == cudaSuccess) err = cudaMemcpy(he.data(), be, 8 * blocks, cudaMemcpyDeviceToHost);
         if (err == cudaSuccess) err = cudaMemcpy(hx.data(), bx, 8 * blocks, cudaMemcpyDeviceToHost);
-        cudaFree(arena);
+        device_free(arena);
         GN_CK(err);
         double best = INFINITY;
         unsigned long long x = 0;

@@ -210,7 +210,7 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
     cudaStream_t st = nullptr;
     auto release = [&]() {
         if (st) cudaStreamSynchronize(st);
-        if (arena) cudaFree(arena);
+        if (arena) device_free(arena);
         if (st) cudaStreamDestroy(st);
         arena = nullptr;
         st = nullptr;

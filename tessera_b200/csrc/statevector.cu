@@ -357,6 +357,10 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         size_t freeb = 0, totb = 0;
         SV_CK(cudaMemGetInfo(&freeb, &totb));
         const size_t need = dim * (16 + 8 + 8) + (1 << 20);
+        if (need > freeb) {  // the library's own pool may hold some of it
+            device_trim();
+            SV_CK(cudaMemGetInfo(&freeb, &totb));
+        }
         if (need > freeb) throw std::invalid_argument("not enough device memory for the 2^n state");
         cudaStream_t st;
         SV_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
@@ -468,7 +472,7 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         if (err == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
-        cudaFree(arena);
+        device_free(arena);
         cudaStreamDestroy(st);
         SV_CK(err);
         double tot = 0, ee = 0, bp = -1;
