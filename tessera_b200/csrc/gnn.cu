@@ -49,6 +49,153 @@ void set_last_error(const std::string& msg);
 // =====================================================================================
 // exact ground state
 // =====================================================================================
+// E(x) as the reference sums it: the edges in the order given, then the fields.
+__device__ __forceinline__ double ground_energy(unsigned long long x, const double* h, const double* w, const int* ei,
+                                                const int* ej, int n, int m) {
+    double e = 0.0;
+#pragma unroll 8
+    for (int q = 0; q < m; ++q) {
+        const int si = ((x >> ei[q]) & 1ull) ? 1 : -1, sj = ((x >> ej[q]) & 1ull) ? 1 : -1;
+        e -= w[q] * (double)(si * sj);
+    }
+    for (int i = 0; i < n; ++i) e -= h[i] * (((x >> i) & 1ull) ? 1.0 : -1.0);
+    return e;
+}
+
+// CTA-wide first minimum: (energy, pattern) in re[0], rx[0]
+__device__ __forceinline__ void ground_reduce(double best, unsigned long long bx, double* re, unsigned long long* rx) {
+    re[threadIdx.x] = best;
+    rx[threadIdx.x] = bx;
+    __syncthreads();
+    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
+        if ((int)threadIdx.x < o) {
+            const double e2 = re[threadIdx.x + o];
+            const unsigned long long x2 = rx[threadIdx.x + o];
+            if (e2 < re[threadIdx.x] || (e2 == re[threadIdx.x] && x2 < rx[threadIdx.x])) {
+                re[threadIdx.x] = e2;
+                rx[threadIdx.x] = x2;
+            }
+        }
+        __syncthreads();
+    }
+}
+
+// The scan for n >= GS_MIN: a thread takes the 2^8 patterns that share their upper bits.  With the
+// upper spins fixed, E = A + B(low) + T(low), where B is the low spins' own couplings (one table of
+// 256 for everybody) and T their fields from above, which splits into two tables of 16, one per
+// half of the low bits: two additions and a comparison per pattern instead of a walk over all
+// edges.  A and T come from the dense coupling matrix.  That sum rounds otherwise than the reference's, so it only picks candidates: pass 0
+// keeps the least sum per CTA, pass 1 revisits the CTAs that hold one within `slack` (twice the
+// two sums' rounding bound) of the least overall and takes the reference's sum of every pattern
+// that close; its first minimum is the answer, as before.
+// Bound: a thread's set-up from the couplings, and at this size the call's own copies.  n = 22, 115
+// edges: 14 + 43 us for the two passes against 400 us for the walk over all edges.
+constexpr int GS_LOW = 8;
+constexpr int GS_MIN = 16;  // patterns of one full CTA: 2^16
+constexpr int GS_NT = 256;
+__global__ void __launch_bounds__(GS_NT) k_ground_scan(const double* h, const int* ei, const int* ej, const double* w,
+                                                       const double* J, double loops, int n, int m, int pass,
+                                                       double slack, double* blk_min, unsigned long long* least,
+                                                       double* blk_e, unsigned long long* blk_x) {
+    __shared__ double low[1 << GS_LOW];
+    __shared__ double re[GS_NT];
+    __shared__ unsigned long long rx[GS_NT];
+    __shared__ double sj[32 * 32], sh[32];  // symmetric couplings (row stride n, zero diagonal), fields
+    const int tid = threadIdx.x;
+    for (int t = tid; t < n * n; t += GS_NT) sj[t] = J[t];
+    if (tid < n) sh[tid] = h[tid];
+    __syncthreads();
+    auto spin = [](unsigned long long x, int i) { return ((x >> i) & 1ull) ? 1.0 : -1.0; };
+    {
+        double b = 0.0;  // couplings among the low spins
+        for (int i = 0; i < GS_LOW; ++i)
+            for (int j = i + 1; j < GS_LOW; ++j) b -= sj[i * n + j] * (spin(tid, i) * spin(tid, j));
+        low[tid] = b;
+    }
+    __syncthreads();
+    const unsigned long long chunks = 1ull << (n - GS_LOW - 8);  // chunks of 2^16 patterns
+    // least: the smallest sum so far as an ordered integer
+    const unsigned long long lk = pass ? *least : 0ull;
+    const double cut = pass ? __longlong_as_double((lk >> 63) ? (long long)(lk ^ (1ull << 63)) : (long long)~lk) + slack
+                            : 0.0;
+    double best = INFINITY;
+    unsigned long long bx = ~0ull;
+    for (unsigned long long c = blockIdx.x; c < chunks; c += gridDim.x) {
+        if (pass && !(blk_min[c] <= cut)) continue;
+        const unsigned long long hi = (c << 16) | ((unsigned long long)tid << GS_LOW);
+        double A = -loops, f[GS_LOW];
+#pragma unroll
+        for (int b = 0; b < GS_LOW; ++b) f[b] = sh[b];
+        for (int i = GS_LOW; i < n; ++i) {
+            const double si = spin(hi, i);
+            const double* row = sj + i * n;
+            double g = sh[i];
+            for (int j = GS_LOW; j < i; ++j) g = fma(row[j], spin(hi, j), g);
+            A = fma(-si, g, A);
+#pragma unroll
+            for (int b = 0; b < GS_LOW; ++b) f[b] = fma(row[b], si, f[b]);
+        }
+        // T of the lower and of the upper four low bits; A goes with the upper
+        auto upper = [&](int u) {
+            double x = A;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) x -= ((u >> b) & 1) ? f[4 + b] : -f[4 + b];
+            return x;
+        };
+        auto lower = [&](int v) {
+            double x = 0.0;
+#pragma unroll
+            for (int b = 0; b < 4; ++b) x -= ((v >> b) & 1) ? f[b] : -f[b];
+            return x;
+        };
+        if (!pass) {
+            double t0[16], mn = INFINITY, mn2 = INFINITY;
+#pragma unroll
+            for (int v = 0; v < 16; ++v) t0[v] = lower(v);
+#pragma unroll 1  // one turn of 16 patterns: the unrolled 256 would not fit the instruction cache
+            for (int u = 0; u < 16; ++u) {
+                const double x = upper(u);
+#pragma unroll
+                for (int v = 0; v < 16; v += 2) {
+                    mn = fmin(mn, x + (t0[v] + low[16 * u + v]));
+                    mn2 = fmin(mn2, x + (t0[v + 1] + low[16 * u + v + 1]));
+                }
+            }
+            mn = fmin(mn, mn2);
+            re[tid] = mn;
+            __syncthreads();
+            for (int o = GS_NT / 2; o > 0; o >>= 1) {
+                if (tid < o) re[tid] = fmin(re[tid], re[tid + o]);
+                __syncthreads();
+            }
+            if (tid == 0) {
+                blk_min[c] = re[0];
+                const long long k = __double_as_longlong(re[0]);
+                atomicMin(least, k < 0 ? (unsigned long long)~k : (unsigned long long)k | (1ull << 63));
+            }
+            __syncthreads();
+        } else {
+#pragma unroll 1
+            for (int l = 0; l < 1 << GS_LOW; ++l)
+                if (upper(l >> 4) + (lower(l & 15) + low[l]) <= cut) {
+                    const unsigned long long x = hi | (unsigned)l;
+                    const double e = ground_energy(x, h, w, ei, ej, n, m);
+                    if (e < best || (e == best && x < bx)) {
+                        best = e;
+                        bx = x;
+                    }
+                }
+        }
+    }
+    if (pass) {
+        ground_reduce(best, bx, re, rx);
+        if (tid == 0) {
+            blk_e[blockIdx.x] = re[0];
+            blk_x[blockIdx.x] = rx[0];
+        }
+    }
+}
+
 __global__ void k_ground(const double* h, const int* ei, const int* ej, const double* w, int n, int m,
                          unsigned long long total, double* blk_e, unsigned long long* blk_x) {
     extern __shared__ double sh[];
@@ -67,12 +214,7 @@ __global__ void k_ground(const double* h, const int* ei, const int* ej, const do
     unsigned long long bx = ~0ull;
     for (unsigned long long x = blockIdx.x * (unsigned long long)blockDim.x + threadIdx.x; x < total;
          x += (unsigned long long)gridDim.x * blockDim.x) {
-        double e = 0.0;
-        for (int q = 0; q < m; ++q) {
-            const int si = ((x >> sh_i[q]) & 1ull) ? 1 : -1, sj = ((x >> sh_j[q]) & 1ull) ? 1 : -1;
-            e -= sh_w[q] * (double)(si * sj);
-        }
-        for (int i = 0; i < n; ++i) e -= sh_h[i] * (((x >> i) & 1ull) ? 1.0 : -1.0);
+        const double e = ground_energy(x, sh_h, sh_w, sh_i, sh_j, n, m);
         if (e < best || (e == best && x < bx)) {
             best = e;
             bx = x;
@@ -80,20 +222,7 @@ __global__ void k_ground(const double* h, const int* ei, const int* ej, const do
     }
     __shared__ double re[256];
     __shared__ unsigned long long rx[256];
-    re[threadIdx.x] = best;
-    rx[threadIdx.x] = bx;
-    __syncthreads();
-    for (int o = blockDim.x / 2; o > 0; o >>= 1) {
-        if ((int)threadIdx.x < o) {
-            const double e2 = re[threadIdx.x + o];
-            const unsigned long long x2 = rx[threadIdx.x + o];
-            if (e2 < re[threadIdx.x] || (e2 == re[threadIdx.x] && x2 < rx[threadIdx.x])) {
-                re[threadIdx.x] = e2;
-                rx[threadIdx.x] = x2;
-            }
-        }
-        __syncthreads();
-    }
+    ground_reduce(best, bx, re, rx);
     if (threadIdx.x == 0) {
         blk_e[blockIdx.x] = re[0];
         blk_x[blockIdx.x] = rx[0];
@@ -738,38 +867,63 @@ double tessera_qa_exact_ground(const double* h, size_t n, const size_t* ei, cons
         GN_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         unsigned long long blocks = (total + 255) / 256;
         if (blocks > (unsigned long long)nsm * 8) blocks = (unsigned long long)nsm * 8;
+        // n >= GS_MIN: the table scan, which needs finite weights for its candidate bound
+        double span = 0.0;
+        for (size_t e = 0; e < m; ++e) span += std::fabs(ew[e]);
+        for (size_t i = 0; i < n; ++i) span += std::fabs(h[i]);
+        const bool scan = n >= GS_MIN && std::isfinite(span);
+        // either sum is within (m + n + 16) roundings of `span` of the true value
+        const double slack = 4.0 * (double)(m + n + 16) * 2.3e-16 * span;
+        const unsigned long long chunks = scan ? 1ull << (n - 16) : 0;
+        if (scan) blocks = std::min<unsigned long long>(chunks, (unsigned long long)nsm * 2);
+        auto al = [](size_t sz) { return (sz + 63) & ~(size_t)63; };
+        // one upload: h, w, ei, ej (and the least sum's start); one download: every CTA's energy
+        // and pattern
+        const size_t o_w = al(8 * n), o_i = o_w + al(8 * m), o_j = o_i + al(4 * m), o_l = o_j + al(4 * m);
+        const size_t o_d = o_l + 64, in_bytes = o_d + (scan ? 8 * n * n : 0), o_e = in_bytes, o_x = o_e + 8 * blocks, o_m = al(o_x + 8 * blocks);
         char* arena = nullptr;
-        const size_t mm = std::max<size_t>(m, 1);
-        const size_t bytes = 64 * 8 + 8 * n + 8 * mm + 8 * mm + 16 * blocks;
-        GN_CK(device_alloc((void**)&arena, bytes));
-        size_t off = 0;
-        auto take = [&](size_t sz) {
-            void* r = arena + off;
-            off += (sz + 63) & ~(size_t)63;
-            return r;
-        };
-        double* dh = (double*)take(8 * n);
-        double* dw = (double*)take(8 * mm);
-        int* di = (int*)take(4 * mm);
-        int* dj = (int*)take(4 * mm);
-        double* be = (double*)take(8 * blocks);
-        unsigned long long* bx = (unsigned long long*)take(8 * blocks);
-        cudaError_t err = cudaMemcpy(dh, h, 8 * n, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess && m) err = cudaMemcpy(dw, ew, 8 * m, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess && m) err = cudaMemcpy(di, a.data(), 4 * m, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess && m) err = cudaMemcpy(dj, b.data(), 4 * m, cudaMemcpyHostToDevice);
-        if (err == cudaSuccess && smem > 48 * 1024)
+        GN_CK(device_alloc((void**)&arena, o_m + al(8 * std::max<unsigned long long>(chunks, 1))));
+        std::vector<char> up(in_bytes, (char)0xff), down(16 * blocks);
+        std::memcpy(up.data(), h, 8 * n);
+        if (m) {
+            std::memcpy(up.data() + o_w, ew, 8 * m);
+            std::memcpy(up.data() + o_i, a.data(), 4 * m);
+            std::memcpy(up.data() + o_j, b.data(), 4 * m);
+        }
+        double loops = 0.0;  // self-loops add a constant
+        if (scan) {
+            double* J = (double*)(up.data() + o_d);
+            std::fill(J, J + n * n, 0.0);
+            for (size_t e = 0; e < m; ++e) {
+                if (a[e] == b[e]) loops += ew[e];
+                else J[a[e] * n + b[e]] += ew[e], J[b[e] * n + a[e]] += ew[e];
+            }
+        }
+        double *dh = (double*)arena, *dw = (double*)(arena + o_w);
+        int *di = (int*)(arena + o_i), *dj = (int*)(arena + o_j);
+        unsigned long long* dl = (unsigned long long*)(arena + o_l);
+        double* be = (double*)(arena + o_e);
+        unsigned long long* bx = (unsigned long long*)(arena + o_x);
+        double* bm = (double*)(arena + o_m);
+        cudaError_t err = cudaMemcpy(arena, up.data(), in_bytes, cudaMemcpyHostToDevice);
+        if (err == cudaSuccess && !scan && smem > 40 * 1024) {
             err = cudaFuncSetAttribute(k_ground, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        }
         if (err == cudaSuccess) {
-            k_ground<<<(unsigned)blocks, 256, smem>>>(dh, di, dj, dw, (int)n, (int)m, total, be, bx);
+            if (scan) {
+                for (int pass = 0; pass < 2; ++pass)
+                    k_ground_scan<<<(unsigned)blocks, GS_NT>>>(dh, di, dj, dw, (double*)(arena + o_d), loops, (int)n,
+                                                               (int)m, pass, slack, bm, dl, be, bx);
+            } else {
+                k_ground<<<(unsigned)blocks, 256, smem>>>(dh, di, dj, dw, (int)n, (int)m, total, be, bx);
+            }
             err = cudaGetLastError();
         }
-        std::vector<double> he(blocks);
-        std::vector<unsigned long long> hx(blocks);
-        if (err == cudaSuccess) err = cudaMemcpy(he.data(), be, 8 * blocks, cudaMemcpyDeviceToHost);
-        if (err == cudaSuccess) err = cudaMemcpy(hx.data(), bx, 8 * blocks, cudaMemcpyDeviceToHost);
+        if (err == cudaSuccess) err = cudaMemcpy(down.data(), be, 16 * blocks, cudaMemcpyDeviceToHost);
         device_free(arena);
         GN_CK(err);
+        const double* he = (const double*)down.data();
+        const unsigned long long* hx = (const unsigned long long*)(down.data() + 8 * blocks);
         double best = INFINITY;
         unsigned long long x = 0;
         for (unsigned long long k = 0; k < blocks; ++k)
