@@ -100,7 +100,9 @@ typedef struct tessera_qa_config {
                                in a single instance with jacobi_block 0): 0 = default (on), 1 = on, 2 = off.
                                On: a row-pivoted Householder LQ of theta (P^T theta = L Q^H) runs first and
                                the Jacobi works on L, which takes fewer sweeps (Drmac-Veselic
-                               preconditioning); the results are the same up to rounding */
+                               preconditioning); the results are the same up to rounding.  Also before the
+                               Jacobi of complex128 theta held in shared memory (up to 112 rows), where the
+                               LQ stops at theta's numerical rank */
     int reserved[4];
 } tessera_qa_config;
 

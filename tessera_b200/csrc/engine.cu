@@ -674,6 +674,7 @@ public:
         t.pp.rows_cap = rows_cap;
         t.pp.cols_cap = rows_cap;  // theta is at most 2 cap x 2 cap
         t.pp.lq = 0;
+        t.pp.rr = C_.precond != 2 ? 1 : 0;
         t.ent_steps = entc_;
         t.n_ent = n_ent_;
         t.pad = 0;
@@ -965,7 +966,7 @@ private:
             TQ_CK(cudaEventRecord(a, stream_));
         }
         launch_svd<T>(M, i, C_.chi, tol_for(2 * dl), C_.max_sweeps, work(), 2 * dl, 2 * dr, pick_block(2 * dl, 2 * dr),
-                      stream_, 0, 0, lq ? 1 : 0);
+                      stream_, 0, 0, lq ? 1 : 0, C_.precond != 2 ? 1 : 0);
         if (C_.timing) {
             TQ_CK(cudaEventRecord(b, stream_));
             timed_.push_back({a, b});

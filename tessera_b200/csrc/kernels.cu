@@ -349,6 +349,38 @@ __device__ __forceinline__ bool jacobi_rotation(const double v0, const double v1
     return true;
 }
 
+__device__ __forceinline__ float sqrt_approx(const float x) {
+    float r;
+    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+
+// 1 / sqrt(x) for x in [1, 4): an FP32 start y (relative error 1e-7) and one third-order step
+// y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2 of the series of (1 - e)^(-1/2), which leaves e^3
+__device__ __forceinline__ double rsqrt_near1(const double x) {
+    const double y = (double)rsqrtf((float)x);
+    const double e = fma(-x, y * y, 1.0);
+    return fma(y * e, fma(0.375, e, 0.5), y);
+}
+
+// tau = t e of the rotation w_p <- c (w_p - conj(tau) w_q), w_q <- c (w_q + tau w_p), from
+// alpha = |w_p|^2, beta = |w_q|^2, gamma = w_p^H w_q; false when the pair is converged or frozen.
+__device__ __forceinline__ bool jacobi_tau(const double a, const double b, const double gr, const double gi,
+                                           const double tol2, const double tiny, const bool mixed, double& tr,
+                                           double& ti) {
+    const double g2 = fma(gr, gr, gi * gi);
+    if (!(pair_live(a, b, tiny, mixed) && g2 > tol2 * (a * b))) return false;
+    // 2^-exponent(max(a, b)): the scaled values fit FP32 (|gamma| >= 1e-13 sqrt(a b) >= 1e-30 max)
+    const int e = (__double2hiint(fmax(a, b)) >> 20) & 0x7ff;
+    const double f = __hiloint2double((2046 - e) << 20, 0);
+    const float d = (float)((b - a) * f), xr = (float)(gr * f), xi = (float)(gi * f);
+    const float h = sqrt_approx(fmaf(d, d, 4.f * fmaf(xr, xr, xi * xi)));
+    const float s = __fdividef(d >= 0.f ? 2.f : -2.f, fabsf(d) + h);
+    tr = (double)(xr * s);
+    ti = (double)(xi * s);
+    return true;
+}
+
 // Per-lane partial sums of alpha = |x|^2, beta = |y|^2 and gamma = x^H y over the rows a lane
 // holds, for complex64: FP32 products summed in FP32 over the lane's rows (at most 16 in every
 // kernel here, relative error about 1e-6, under the complex64 convergence tolerance
@@ -892,6 +924,237 @@ __device__ void jacobi_core(cplx_t<T>* col, const int rc, const int R, const int
     __syncthreads();
 }
 
+// ------------------------------------------------------------------------------------
+// Resident complex128: a rank-revealing pivoted LQ of the matrix in shared memory, then the same
+// circle-method Jacobi on the columns that are left.
+//
+// P^T W = L Q^H (lq.cu has the why): the Jacobi runs on P L, whose columns are few and nearly in
+// order.  The factorisation stops when what is left of W weighs no more than 1e-6 of the noise
+// floor on |w|^2, the weight under which the Jacobi leaves a column alone for good (pair_live), so a
+// bond of numerical rank r costs r (r - 1) / 2 pairs a sweep instead of N (N - 1) / 2.  On theta of
+// the n = 16 chain at chi = 32 (mean 31 columns, rank 21) a numpy model takes 138 rounds instead of
+// 518, on dense n = 10 instances 50 instead of 189.  Measured, whole calls: that chain's first 40
+// steps 261 -> 86 ms, 160 dense instances of n 8-10 373 -> 233 ms, the n = 6 anneal 18.6 -> 11.1 ms.
+// Bound: the chain of a step (pivot, reflector, products, barrier, update, barrier) and of a round.
+//
+// Threads are a grid of parts x rows (a part is whole warps): a thread takes the columns of its
+// part of one row.  Step k: every warp picks the unpivoted row of largest remaining norm for
+// itself from the norms the last step left; its products w = X u^H by parts; a barrier; X -= tau w u
+// and the new norms by parts; a barrier.  Returns the number of columns; nothing when the CTA has
+// fewer threads than rows (the caller's launch shape excludes it).
+// ------------------------------------------------------------------------------------
+constexpr int RLQ_ROWS = 128;  // rows a resident complex128 theta can have (112), in whole warps
+
+constexpr int RLQ_CELLS = 256;  // threads of the parts x rows grid
+
+struct RlqShared {
+    double nrm[RLQ_CELLS];   // [part][row]: the rows' remaining squared norms
+    double2 w[RLQ_CELLS];    // [part][row]: the rows' products with the reflector
+    unsigned char piv[RLQ_ROWS];
+};
+
+__device__ int lq_resident(double2* col, const int rc, const int R, const int N, const double tiny, RlqShared& sh) {
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int Rp = (R + 31) & ~31;
+    const int parts = (blockDim.x < RLQ_CELLS ? blockDim.x : RLQ_CELLS) / Rp;
+    if (parts < 1 || R > RLQ_ROWS) return N;
+    const int row = tid % Rp, part = tid / Rp;
+    const bool mine = row < R && part < parts;
+    if (tid < RLQ_ROWS) sh.piv[tid] = tid < R ? 0 : 1;
+    if (part < parts) {
+        double nz = 0.0;
+        if (mine)
+            for (int c = part; c < N; c += parts) {
+                const double2 x = col[c * rc + row];
+                nz = fma(x.x, x.x, fma(x.y, x.y, nz));
+            }
+        sh.nrm[tid] = nz;
+    }
+    __syncthreads();
+    const int kmax = R < N ? R : N;
+    int k = 0;
+    for (; k < kmax; ++k) {
+        // the pivot row, by every warp alike: largest remaining norm, lowest row on ties
+        double best = -1.0, left = 0.0;
+        int p = RLQ_ROWS;
+        for (int r = lane; r < R; r += 32)
+            if (!sh.piv[r]) {
+                double v = 0.0;
+                for (int q = 0; q < parts; ++q) v += sh.nrm[q * Rp + r];
+                left += v;
+                if (v > best) { best = v; p = r; }
+            }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const double b2 = __shfl_xor_sync(0xffffffffu, best, o);
+            const int p2 = __shfl_xor_sync(0xffffffffu, p, o);
+            left += __shfl_xor_sync(0xffffffffu, left, o);
+            if (b2 > best || (b2 == best && p2 < p)) { best = b2; p = p2; }
+        }
+        if (left != left) return N;  // not a number: every column stays in, and raises the status
+        if (!(left > 1e-6 * tiny) || !(best > 0.0)) break;
+        // reflector u = (e (|x_0| + alpha), x_1, ...) of that row's columns >= k
+        const double2 x0 = col[k * rc + p];
+        const double alpha = sqrt(best), m0 = sqrt(fma(x0.x, x0.x, x0.y * x0.y));
+        const double im = m0 > 0.0 ? 1.0 / m0 : 0.0;
+        const double2 e0 = m0 > 0.0 ? make_double2(x0.x * im, x0.y * im) : make_double2(1.0, 0.0);
+        const double2 u0 = make_double2(e0.x * (m0 + alpha), e0.y * (m0 + alpha));
+        const double tau = 1.0 / (alpha * (alpha + m0));
+        const bool live = mine && row != p && !sh.piv[row];
+        const int c1 = k + 1 + part;  // this thread's columns: k (part 0), then k + 1 + part, ...
+        if (live) {
+            double2 a = make_double2(0.0, 0.0), b = make_double2(0.0, 0.0);
+            if (part == 0) cfma_conj(a, u0, col[k * rc + row]);
+            int c = c1;
+            for (; c + parts < N; c += 2 * parts) {
+                cfma_conj(a, col[c * rc + p], col[c * rc + row]);
+                cfma_conj(b, col[(c + parts) * rc + p], col[(c + parts) * rc + row]);
+            }
+            if (c < N) cfma_conj(a, col[c * rc + p], col[c * rc + row]);
+            sh.w[tid] = make_double2(a.x + b.x, a.y + b.y);
+        }
+        __syncthreads();
+        if (live) {
+            double2 w = make_double2(0.0, 0.0);
+            for (int q = 0; q < parts; ++q) {
+                w.x += sh.w[q * Rp + row].x;
+                w.y += sh.w[q * Rp + row].y;
+            }
+            w.x *= -tau;
+            w.y *= -tau;
+            if (part == 0) cfma(col[k * rc + row], w, u0);
+            double n0 = 0.0, n1 = 0.0;
+            for (int c = c1; c < N; c += parts) {
+                double2 z = col[c * rc + row];
+                cfma(z, w, col[c * rc + p]);
+                col[c * rc + row] = z;
+                n0 = fma(z.x, z.x, n0);
+                n1 = fma(z.y, z.y, n1);
+            }
+            sh.nrm[tid] = n0 + n1;
+        }
+        if (tid == 0) sh.piv[p] = 1;
+        __syncthreads();
+        // the pivot row takes its diagonal entry and zeros to its right (no one reads it again)
+        if (mine && row == p) {
+            if (part == 0) col[k * rc + row] = make_double2(-e0.x * alpha, -e0.y * alpha);
+            for (int c = c1; c < N; c += parts) col[c * rc + row] = make_double2(0.0, 0.0);
+        }
+    }
+    __syncthreads();
+    return k < 1 ? 1 : k;
+}
+
+// One sweep-by-sweep circle-method Jacobi in shared memory with LPP lanes per pair (R <= 32 RPL / ...):
+// as jacobi_core, with the angle of jacobi_tau.
+template <int LPP, int RPL>
+__device__ void jacobi_core_d(double2* col, const int rc, const int R, const int N, const double tol,
+                              const double tiny, const int max_sweeps, int* s_rot, int& sweeps, bool& converged,
+                              double& rotations) {
+    constexpr int PPW = 32 / LPP;
+    const int tid = threadIdx.x, NW = blockDim.x >> 5, warp = tid >> 5, lane = tid & 31;
+    const int sub = lane / LPP, sl = lane % LPP;
+    const int Nc = N + (N & 1);
+    const int npairs = Nc / 2;
+    const double tol2 = tol * tol;
+    if (tid == 0) {
+        s_rot[0] = 0;
+        s_rot[1] = 0;
+    }
+    __syncthreads();
+    int sweep = 0;
+    converged = false;
+    rotations = 0.0;
+    bool mixed = true;
+    for (; sweep < max_sweeps; ++sweep) {
+        int rot = 0;
+        for (int r = 0; r < Nc - 1; ++r) {
+            for (int base = warp * PPW; base < npairs; base += NW * PPW) {  // warp-uniform
+                const int pr = base + sub;
+                int p = N, q = N;
+                if (pr < npairs) tournament(Nc, r, pr, p, q);
+                const bool ok = p < N && q < N;
+                double2* cp = col + (ok ? p : 0) * rc + sl;
+                double2* cq = col + (ok ? q : 0) * rc + sl;
+                double2 x[RPL], y[RPL];
+#pragma unroll
+                for (int k = 0; k < RPL; ++k) {
+                    const bool in = ok && sl + LPP * k < R;
+                    x[k] = in ? cp[LPP * k] : make_double2(0.0, 0.0);
+                    y[k] = in ? cq[LPP * k] : make_double2(0.0, 0.0);
+                }
+                double a = 0.0, b = 0.0, gr = 0.0, gi = 0.0;
+#pragma unroll
+                for (int k = 0; k < RPL; ++k) {
+                    a = fma(x[k].x, x[k].x, fma(x[k].y, x[k].y, a));
+                    b = fma(y[k].x, y[k].x, fma(y[k].y, y[k].y, b));
+                    gr = fma(x[k].x, y[k].x, fma(x[k].y, y[k].y, gr));
+                    gi = fma(x[k].x, y[k].y, fma(-x[k].y, y[k].x, gi));
+                }
+#pragma unroll
+                for (int o = LPP / 2; o > 0; o >>= 1) {
+                    a += __shfl_xor_sync(0xffffffffu, a, o);
+                    b += __shfl_xor_sync(0xffffffffu, b, o);
+                    gr += __shfl_xor_sync(0xffffffffu, gr, o);
+                    gi += __shfl_xor_sync(0xffffffffu, gi, o);
+                }
+                double tr, ti;
+                if (ok && jacobi_tau(a, b, gr, gi, tol2, tiny, mixed, tr, ti)) {
+                    const double c = rsqrt_near1(fma(tr, tr, fma(ti, ti, 1.0)));
+                    tr *= c;
+                    ti *= c;
+#pragma unroll
+                    for (int k = 0; k < RPL; ++k) {
+                        const double2 u = x[k], v = y[k];
+                        if (sl + LPP * k < R) {
+                            // x' = c (x - conj(tau) y), y' = c (y + tau x)
+                            cp[LPP * k] = make_double2(fma(-ti, v.y, fma(-tr, v.x, c * u.x)),
+                                                       fma(ti, v.x, fma(-tr, v.y, c * u.y)));
+                            cq[LPP * k] = make_double2(fma(-ti, u.y, fma(tr, u.x, c * v.x)),
+                                                       fma(ti, u.x, fma(tr, u.y, c * v.y)));
+                        }
+                    }
+                    if (sl == 0) ++rot;
+                }
+            }
+            __syncthreads();
+        }
+        if (rot) atomicAdd(&s_rot[sweep & 1], rot);
+        __syncthreads();
+        const int done = s_rot[sweep & 1];
+        if (tid == 0) s_rot[(sweep + 1) & 1] = 0;
+        rotations += done;
+        if (done == 0) {
+            converged = true;
+            ++sweep;
+            break;
+        }
+        mixed = still_mixed(mixed, done, N, sweep);
+    }
+    sweeps = sweep;
+    __syncthreads();
+}
+
+// The resident Jacobi of a class (LPP lanes per pair hold its rows): complex64 always with LPP
+// lanes; complex128 with more lanes a pair where that still takes every pair in one turn, since a
+// round then lasts as long as one pair's chain (loads, products, reduction, angle, update).
+template <typename T, int LPP>
+__device__ __forceinline__ void resident_jacobi(cplx_t<T>* col, const int rc, const int R, const int N,
+                                                const double tol, const double tiny, const int max_sweeps, int* s_rot,
+                                                int& sweeps, bool& converged, double& rotations) {
+    if constexpr (sizeof(T) == 4) {
+        jacobi_core<T, LPP>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
+    } else {
+        const int npairs = (N + 1) / 2, NT = blockDim.x;
+        if (npairs * 32 <= NT)
+            jacobi_core_d<32, LPP / 4>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
+        else if (LPP <= 16 && npairs * 16 <= NT)
+            jacobi_core_d<16, LPP / 2>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
+        else
+            jacobi_core_d<LPP, 8>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
+    }
+}
+
 // sum of |w|^2 over an R x N shared-memory matrix, returned to every thread
 template <typename T>
 __device__ double block_fro2(const cplx_t<T>* col, const int rc, const int R, const int N, double* red) {
@@ -936,6 +1199,22 @@ __device__ void resident_norms(const cplx_t<T>* col, const int rc, const int R, 
     __syncthreads();
 }
 
+// Columns the resident Jacobi works on: complex128 with rr, those of the rank-revealing LQ (the
+// others' squared norms become zero); else all N.
+template <typename T>
+__device__ __forceinline__ int resident_rank(cplx_t<T>* col, const int rc, const int R, const int N, const double tiny,
+                                             const int rr, double* sig2) {
+    if constexpr (sizeof(T) == 8) {
+        if (rr) {
+            __shared__ RlqShared lqs;
+            const int r = lq_resident(col, rc, R, N, tiny, lqs);
+            for (int e = r + threadIdx.x; e < N; e += blockDim.x) sig2[e] = 0.0;
+            return r;
+        }
+    }
+    return N;
+}
+
 __device__ __forceinline__ double noise_tiny(double pp_tiny, int R, double fro2, bool single) {
     const double ulp = single ? 1.1920928955078125e-07 : 2.220446049250313e-16;
     const double floor_rel = 8.0 * sqrt((double)R) * ulp;
@@ -970,9 +1249,10 @@ __device__ void svd_resident_body(const MpsView<T>& mps, const SvdWork<T>& wk, c
     int sweep = 0;
     bool converged = false;
     double rots = 0.0;
-    jacobi_core<T, LPP>(col, rc, R, N, pp.tol, tiny, pp.max_sweeps, s_rot, sweep, converged, rots);
-    resident_norms<T>(col, rc, R, N, wk.W, ld, wk.sig2);
-    const double flops = (double)sweep * 0.5 * N * (N - 1) * R * 16.0 + rots * R * 32.0;
+    const int Nr = resident_rank<T>(col, rc, R, N, tiny, pp.rr && !pp.no_trunc, wk.sig2);
+    resident_jacobi<T, LPP>(col, rc, R, Nr, pp.tol, tiny, pp.max_sweeps, s_rot, sweep, converged, rots);
+    resident_norms<T>(col, rc, R, Nr, wk.W, ld, wk.sig2);
+    const double flops = (double)sweep * 0.5 * Nr * (Nr - 1) * R * 16.0 + rots * R * 32.0;
     svd_finish<T>(mps, wk, pp, R, N, fmax(1e-28, tiny), sweep, converged, 2.0 * (double)R * N * sizeof(V), smraw,
                   red, flops);
 }
@@ -1064,13 +1344,14 @@ __device__ void resident_update(const MpsView<T>& mps, const ScheduleView& sch, 
     int sweep = 0;
     bool converged = false;
     double rots = 0.0;
-    jacobi_core<T, LPP>(col, rc, R, N, pp0.tol, tiny, pp0.max_sweeps, s_rot, sweep, converged, rots);
-    resident_norms<T>(col, rc, R, N, nullptr, ld, wk.sig2);
+    const int Nr = resident_rank<T>(col, rc, R, N, tiny, pp0.rr, wk.sig2);
+    resident_jacobi<T, LPP>(col, rc, R, Nr, pp0.tol, tiny, pp0.max_sweeps, s_rot, sweep, converged, rots);
+    resident_norms<T>(col, rc, R, Nr, nullptr, ld, wk.sig2);
     SvdParams pp = pp0;
     pp.bond = i;
     // global traffic of the update: A and C read, theta written and read back, A' and C' written
     const double bytes = (double)sizeof(V) * (2.0 * dl * mid + 2.0 * mid * dr + 3.0 * R * N);
-    const double flops = (double)sweep * 0.5 * N * (N - 1) * R * 16.0 + rots * R * 32.0;
+    const double flops = (double)sweep * 0.5 * Nr * (Nr - 1) * R * 16.0 + rots * R * 32.0;
     svd_finish<T>(mps, wk, pp, R, N, fmax(1e-28, tiny), sweep, converged, bytes, sortbuf, red, flops);
     __syncthreads();
     const int keep = mps.dims[i + 1];
@@ -1182,6 +1463,7 @@ static void res_launch(const MpsView<T>* mps, const SvdWork<T>* wk, const SvdPar
     const int pairs = pp.cols_cap / 2;
     const int warps = (pairs + (32 / LPP) - 1) / (32 / LPP);
     int nt = 32 * (warps < 1 ? 1 : warps);
+    if (sizeof(T) == 8 && nt < 256) nt = 256;  // the LQ: a thread for every row, twice over
     if (nt > RES_MAXT) nt = RES_MAXT;
     if (insts) {
         auto fn = k_svd_res_batch<T, LPP>;
@@ -1977,38 +2259,6 @@ __device__ void svd_body_rc(const MpsView<T>& mps, const SvdWork<T>& wk, const S
 // ------------------------------------------------------------------------------------
 constexpr int RCD_MAXN = 512;  // columns (2^-511 is the least a scale can reach within a sweep)
 
-__device__ __forceinline__ float sqrt_approx(const float x) {
-    float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
-// 1 / sqrt(x) for x in [1, 4): an FP32 start y (relative error 1e-7) and one third-order step
-// y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2 of the series of (1 - e)^(-1/2), which leaves e^3
-__device__ __forceinline__ double rsqrt_near1(const double x) {
-    const double y = (double)rsqrtf((float)x);
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
-// tau = t e of the rotation w_p <- c (w_p - conj(tau) w_q), w_q <- c (w_q + tau w_p), from
-// alpha = |w_p|^2, beta = |w_q|^2, gamma = w_p^H w_q; false when the pair is converged or frozen.
-__device__ __forceinline__ bool jacobi_tau(const double a, const double b, const double gr, const double gi,
-                                           const double tol2, const double tiny, const bool mixed, double& tr,
-                                           double& ti) {
-    const double g2 = fma(gr, gr, gi * gi);
-    if (!(pair_live(a, b, tiny, mixed) && g2 > tol2 * (a * b))) return false;
-    // 2^-exponent(max(a, b)): the scaled values fit FP32 (|gamma| >= 1e-13 sqrt(a b) >= 1e-30 max)
-    const int e = (__double2hiint(fmax(a, b)) >> 20) & 0x7ff;
-    const double f = __hiloint2double((2046 - e) << 20, 0);
-    const float d = (float)((b - a) * f), xr = (float)(gr * f), xi = (float)(gi * f);
-    const float h = sqrt_approx(fmaf(d, d, 4.f * fmaf(xr, xr, xi * xi)));
-    const float s = __fdividef(d >= 0.f ? 2.f : -2.f, fabsf(d) + h);
-    tr = (double)(xr * s);
-    ti = (double)(xi * s);
-    return true;
-}
-
 // scale of a column (W = d X) and its reciprocal, after a rotation with cosine c: i = 1 / d kept to
 // rounding by one Newton step
 struct ColScale {
@@ -2541,9 +2791,10 @@ static int svd_launch_bw(const MpsView<T>& mps, const SvdParams& pp, SvdWork<T> 
 
 template <typename T>
 int launch_svd(const MpsView<T>& mps, int bond, int chi, double tol, int max_sweeps, SvdWork<T> wk,
-               int rows_ub, int cols_ub, int block_w, cudaStream_t s, int R, int N, int lq) {
+               int rows_ub, int cols_ub, int block_w, cudaStream_t s, int R, int N, int lq, int rr) {
     SvdParams pp{};
     pp.lq = lq;
+    pp.rr = rr;
     pp.bond = bond;
     pp.R = R;
     pp.N = N;
@@ -3192,7 +3443,7 @@ void launch_entropy_batch(const InstTask<T>* insts, int ninst, cudaStream_t s) {
     template void launch_theta<T>(const MpsView<T>&, const ScheduleView&, GateOp, const double*, SvdWork<T>, \
                                   int, int, cudaStream_t);                                                  \
     template int launch_svd<T>(const MpsView<T>&, int, int, double, int, SvdWork<T>, int, int, int,         \
-                               cudaStream_t, int, int, int);                                                \
+                               cudaStream_t, int, int, int, int);                                           \
     template void launch_absorb<T>(const MpsView<T>&, int, SvdWork<T>, int, int, int, cudaStream_t);        \
     template void launch_chain<T>(const MpsView<T>&, int, const ChainStep*, int, cplx_t<T>*, cplx_t<T>*,   \
                                   GridBar*, RunStats*, int, cudaStream_t);                                  \

@@ -47,3 +47,25 @@ def test_update_matches_numpy(count, chi, block):
         iso = a.reshape(-1, a.shape[2])
         assert np.linalg.norm(iso.conj().T @ iso - np.eye(a.shape[2])) < 1e-11
     s.close()
+
+
+@pytest.mark.parametrize("n,chi,dmax", [(2, 2, 1), (3, 3, 2), (5, 4, 2), (8, 5, 1), (9, 16, 2), (10, 17, 1),
+                                        (10, 32, 2), (11, 32, 1), (12, 47, 1), (12, 56, 1)])
+def test_rank_revealing_lq_leaves_the_anneal_alone(n, chi, dmax):
+    """Small theta with and without the LQ in front of the resident Jacobi, from a product state (rank 1)
+    through growing ranks, wide and tall theta at the ends of the chain.  <H>, <Z> and the entropy agree to
+    1e-9, a thousand updates' worth of rounding at 1e-12, plus what truncation amplifies: ten times the
+    change that 4 ulps on the inputs make to the run without the LQ."""
+    p = instances.chain_range(n=n, dmax=dmax, seed=n, T=0.8, dt=0.1, chi=chi, hzero=False)
+
+    def run(precondition, eps=0.0):
+        r = ffi.anneal(p.h * (1 + eps), p.ei, p.ej, p.ew * (1 + eps), p.sa, p.sb * (1 + eps), dt=p.dt, chi=chi,
+                       jacobi_precondition=precondition)
+        assert r.status == 0
+        return [np.atleast_1d(x) for x in (r.expected_energy, r.z_expect, r.entropy, r.norm2, r.max_trunc)]
+
+    ref = run(2)
+    moved = [run(2, eps) for eps in (4e-16, -4e-16, 8e-16)]
+    for k, (x, y) in enumerate(zip(run(0), ref)):
+        own = max(np.max(np.abs(m[k] - y)) for m in moved)
+        assert np.max(np.abs(x - y)) < 1e-9 + 10 * own, k
