@@ -484,19 +484,37 @@ public:
     // <Z_i>, <Z_i Z_j>, <psi|psi>, readout, prob (cuda/src/mps.cpp:358-380).
     void observe(tessera_qa_result* r) override {
         const MpsView<T> M = mps();
-        if (!obs_) {  // environments for the final observables, allocated on first use
-            const size_t bytes = sizeof(V) * (size_t)cap_ * cap_ * obs_units_;
-            TQ_CK(device_alloc((void**)&obs_, bytes));
-            TQ_CK(cudaMemsetAsync(obs_, 0, sizeof(V), stream_));
-            V one = mk<V>(1, 0);
-            TQ_CK(cudaMemcpyAsync(obs_, &one, sizeof(V), cudaMemcpyHostToDevice, stream_));
-        }
+        ensure_obs();
         launch_chain<T>(M, 1, obsR_, n_, obs_, xs_, bar_, stats_, cap_, stream_);
         launch_chain<T>(M, 0, obsL_, n_obsL_, obs_, xs_, bar_, stats_, cap_, stream_);
-        launch_pair_dots<T>(M, obs_, dots_, 1 + n_ + m_, dotout_, stream_);
-        std::vector<double> v(1 + n_ + m_);
+        launch_pair_dots<T>(M, obs_, dots_, n_dots(), dotout_, stream_);
+        std::vector<double> v(n_dots());
         TQ_CK(cudaMemcpyAsync(v.data(), dotout_, sizeof(double) * v.size(), cudaMemcpyDeviceToHost, stream_));
         TQ_CK(cudaStreamSynchronize(stream_));
+        std::vector<int8_t> spins(n_);
+        readout(v.data(), spins.data());
+        TQ_CK(cudaMemcpyAsync(spins_d_, spins.data(), n_, cudaMemcpyHostToDevice, stream_));
+        launch_amplitude<T>(M, spins_d_, vbuf_, amp2_, stream_);
+        double a2 = 0;
+        TQ_CK(cudaMemcpyAsync(&a2, amp2_, sizeof(double), cudaMemcpyDeviceToHost, stream_));
+        TQ_CK(cudaStreamSynchronize(stream_));
+        report(v.data(), spins.data(), a2, r);
+    }
+    // environments for the final observables, allocated on first use
+    void ensure_obs() {
+        if (obs_) return;
+        const size_t bytes = sizeof(V) * (size_t)cap_ * cap_ * obs_units_;
+        TQ_CK(device_alloc((void**)&obs_, bytes));
+        TQ_CK(cudaMemsetAsync(obs_, 0, sizeof(V), stream_));
+        V one = mk<V>(1, 0);
+        TQ_CK(cudaMemcpyAsync(obs_, &one, sizeof(V), cudaMemcpyHostToDevice, stream_));
+    }
+    int n_dots() const { return 1 + n_ + m_; }
+    // sign(<Z_i>), ties -> +1, from the closing products (norm, <Z_i>, <Z_i Z_j>)
+    void readout(const double* v, int8_t* spins) const {
+        for (int i = 0; i < n_; ++i) spins[i] = (v[0] > 0 ? v[1 + i] / v[0] : 0.0) >= 0.0 ? 1 : -1;
+    }
+    void report(const double* v, const int8_t* spins, double a2, tessera_qa_result* r) const {
         const double nrm = v[0];
         std::vector<double> ez(n_), ezz(m_);
         for (int i = 0; i < n_; ++i) ez[i] = nrm > 0 ? v[1 + i] / nrm : 0.0;
@@ -504,24 +522,21 @@ public:
         double eexp = 0.0;
         for (int e = 0; e < m_; ++e) eexp -= P_.w[e] * ezz[e];
         for (int i = 0; i < n_; ++i) eexp -= P_.h[i] * ez[i];
-        std::vector<int8_t> spins(n_);
-        for (int i = 0; i < n_; ++i) spins[i] = ez[i] >= 0.0 ? 1 : -1;
         double E = 0.0;
         for (int e = 0; e < m_; ++e) E -= P_.w[e] * spins[P_.ei[e]] * spins[P_.ej[e]];
         for (int i = 0; i < n_; ++i) E -= P_.h[i] * spins[i];
-        TQ_CK(cudaMemcpyAsync(spins_d_, spins.data(), n_, cudaMemcpyHostToDevice, stream_));
-        launch_amplitude<T>(M, spins_d_, vbuf_, amp2_, stream_);
-        double a2 = 0;
-        TQ_CK(cudaMemcpyAsync(&a2, amp2_, sizeof(double), cudaMemcpyDeviceToHost, stream_));
-        TQ_CK(cudaStreamSynchronize(stream_));
         if (r) {
             r->energy = E;
             r->expected_energy = eexp;
             r->prob = nrm > 0 ? a2 / nrm : 0.0;
             r->norm2 = nrm;
-            if (r->spins) std::memcpy(r->spins, spins.data(), n_);
+            if (r->spins) std::memcpy(r->spins, spins, n_);
             if (r->z_expect) std::memcpy(r->z_expect, ez.data(), sizeof(double) * n_);
         }
+    }
+    // this instance's part of a batch's observables (ensure_obs() first)
+    ObsTask<T> obs_task(long long out_off, long long spin_off) const {
+        return ObsTask<T>{mps(), obsR_, obsL_, dots_, obs_, xs_, vbuf_, stats_, n_obsL_, n_dots(), out_off, spin_off};
     }
 
     // `count` basis patterns drawn from |<x|psi>|^2 (K9), their Ising energies on the host
@@ -529,12 +544,7 @@ public:
         if (count == 0) return;
         if (count > (size_t)1 << 24) throw ArgError("at most 2^24 samples per call");
         const MpsView<T> M = mps();
-        if (!obs_) {
-            const size_t bytes = sizeof(V) * (size_t)cap_ * cap_ * obs_units_;
-            TQ_CK(device_alloc((void**)&obs_, bytes));
-            V one = mk<V>(1, 0);
-            TQ_CK(cudaMemcpyAsync(obs_, &one, sizeof(V), cudaMemcpyHostToDevice, stream_));
-        }
+        ensure_obs();
         launch_chain<T>(M, 1, obsR_, n_, obs_, xs_, bar_, stats_, cap_, stream_);
         int8_t* d = nullptr;
         TQ_CK(device_alloc((void**)&d, count * (size_t)n_));
@@ -1265,6 +1275,57 @@ public:
     double ms() const { return ms_; }
     long long launches() const { return launches_; }
 
+    // Whether observe_all() beats one instance after another.  Bonds up to 32: a CTA's chains take
+    // about as long as the cooperative launches of one instance (latency either way), so two
+    // instances are enough; larger bonds, up to 1 ms a product on one SM, want 32 of them (148 at
+    // bond 256: 0.2 s together against 1.2 s in turn).
+    bool observe_together() const { return eng_.size() >= (cap_max_ <= 32 ? 2u : 32u); }
+    // The final observables of the instances for which want[b] is set, in two launches.
+    void observe_all(const std::vector<char>& want, tessera_qa_result* results) {
+        std::vector<ObsTask<T>> tasks;
+        std::vector<int> who;
+        long long ndots = 0, nspins = 0;
+        for (size_t b = 0; b < eng_.size(); ++b) {
+            if (!want[b]) continue;
+            eng_[b]->ensure_obs();
+            TQ_CK(cudaStreamSynchronize(eng_[b]->own_stream()));
+            tasks.push_back(eng_[b]->obs_task(ndots, nspins));
+            who.push_back((int)b);
+            ndots += eng_[b]->n_dots();
+            nspins += eng_[b]->n();
+        }
+        if (who.empty()) return;
+        const int B = (int)who.size();
+        const size_t o_v = align256(sizeof(ObsTask<T>) * B), o_a = o_v + align256(sizeof(double) * ndots);
+        const size_t o_s = o_a + align256(sizeof(double) * B);
+        struct Buf {  // released on every way out
+            char* p = nullptr;
+            cudaStream_t st;
+            ~Buf() {
+                if (p) cudaStreamSynchronize(st);
+                device_free(p);
+            }
+        } buf;
+        buf.st = st_;
+        TQ_CK(device_alloc((void**)&buf.p, o_s + align256(nspins)));
+        ObsTask<T>* dt = reinterpret_cast<ObsTask<T>*>(buf.p);
+        double *dv = reinterpret_cast<double*>(buf.p + o_v), *da = reinterpret_cast<double*>(buf.p + o_a);
+        int8_t* ds = reinterpret_cast<int8_t*>(buf.p + o_s);
+        std::vector<double> v(ndots), a2(B);
+        std::vector<int8_t> spins(nspins);
+        TQ_CK(cudaMemcpyAsync(dt, tasks.data(), sizeof(ObsTask<T>) * B, cudaMemcpyHostToDevice, st_));
+        launch_observe_batch<T>(dt, B, dv, st_);
+        TQ_CK(cudaMemcpyAsync(v.data(), dv, sizeof(double) * ndots, cudaMemcpyDeviceToHost, st_));
+        TQ_CK(cudaStreamSynchronize(st_));
+        for (int k = 0; k < B; ++k) eng_[who[k]]->readout(&v[tasks[k].out_off], &spins[tasks[k].spin_off]);
+        TQ_CK(cudaMemcpyAsync(ds, spins.data(), nspins, cudaMemcpyHostToDevice, st_));
+        launch_amplitude_batch<T>(dt, B, ds, da, st_);
+        TQ_CK(cudaMemcpyAsync(a2.data(), da, sizeof(double) * B, cudaMemcpyDeviceToHost, st_));
+        TQ_CK(cudaStreamSynchronize(st_));
+        for (int k = 0; k < B; ++k)
+            eng_[who[k]]->report(&v[tasks[k].out_off], &spins[tasks[k].spin_off], a2[k], &results[who[k]]);
+    }
+
 private:
     // one Trotter step of every instance: half single-site gates, every gate slot, half
     // single-site gates, the qubit-0 entropy, the step counter
@@ -1342,16 +1403,25 @@ static void run_batch(const std::vector<ProblemHost>& P, const std::vector<Confi
         if (P[b].steps != P[0].steps) throw ArgError("batched instances must share the number of schedule steps");
     if (k0 > k1 || k1 > P[0].steps) throw ArgError("step range outside the schedule");
     be.run(k0, k1);
+    std::vector<tessera_qa_result> rs(results, results + be.size());
+    std::vector<char> want(be.size());
+    for (int b = 0; b < be.size(); ++b) {
+        be.at(b).sync_stats(&rs[b]);
+        rs[b].device_ms = be.ms();
+        rs[b].kernel_launches = be.launches();
+        want[b] = !configs[b].skip_observables;
+    }
+    if (be.observe_together()) {
+        be.observe_all(want, rs.data());
+    } else {
+        for (int b = 0; b < be.size(); ++b)
+            if (want[b]) be.at(b).observe(&rs[b]);
+    }
     for (int b = 0; b < be.size(); ++b) {
         Engine<T>& e = be.at(b);
-        tessera_qa_result r = results[b];
-        e.sync_stats(&r);
-        r.device_ms = be.ms();
-        r.kernel_launches = be.launches();
-        if (!configs[b].skip_observables) e.observe(&r);
-        if (r.entropy) e.copy_entropy(r.entropy, k0, k1);
-        if (r.final_mps) e.save(r.final_mps, r.final_mps_bytes, (unsigned long long)k1);
-        results[b] = r;
+        if (rs[b].entropy) e.copy_entropy(rs[b].entropy, k0, k1);
+        if (rs[b].final_mps) e.save(rs[b].final_mps, rs[b].final_mps_bytes, (unsigned long long)k1);
+        results[b] = rs[b];
     }
 }
 

@@ -162,6 +162,25 @@ void launch_pair_dots(const MpsView<T>& mps, const cplx_t<T>* envs, const PairDo
 template <typename T>
 void launch_amplitude(const MpsView<T>& mps, const int8_t* spins, cplx_t<T>* scratch, double* out_amp2,
                       cudaStream_t s);
+// One instance's observables in a batch (engine.cu: Engine::obs_task).
+template <typename T>
+struct ObsTask {
+    MpsView<T> mps;
+    const ChainStep* right;    // n steps
+    const ChainStep* left;
+    const PairDot* dots;
+    cplx_t<T>* envs;
+    cplx_t<T>* X;
+    cplx_t<T>* vbuf;
+    RunStats* stats;
+    int n_left, n_dots;
+    long long out_off;         // first of this instance's n_dots values
+    long long spin_off;        // first of its n readout spins
+};
+template <typename T>
+void launch_observe_batch(const ObsTask<T>* tasks, int ninst, double* out, cudaStream_t s);
+template <typename T>
+void launch_amplitude_batch(const ObsTask<T>* tasks, int ninst, const int8_t* spins, double* out, cudaStream_t s);
 void launch_step_inc(int* step, cudaStream_t s);
 // batched launchers: `refs` selects (instance, gate) pairs; ub_* are upper bounds over the batch
 template <typename T>
