@@ -115,6 +115,23 @@ __device__ __forceinline__ bool grid_sync(GridBar* bar, int* status, unsigned in
     return s_ok != 0;
 }
 
+// Hand-over flags between the CTAs of a cooperative launch: a counter that only grows.  The wait is
+// bounded like the barrier's.
+__device__ __forceinline__ void flag_release(int* p, int v) {
+    asm volatile("st.release.gpu.global.s32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ bool flag_wait(const int* p, int v, uint64_t budget_ns = 2000000000ull) {
+    int x;
+    asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+    if (x >= v) return true;
+    const uint64_t t0 = globaltimer_ns();
+    for (unsigned spins = 1;; ++spins) {
+        asm volatile("ld.acquire.gpu.global.s32 %0, [%1];" : "=r"(x) : "l"(p) : "memory");
+        if (x >= v) return true;
+        if ((spins & 255u) == 0 && globaltimer_ns() - t0 > budget_ns) return false;
+    }
+}
+
 // ---------------------------------------------------------------------------------
 // mbarrier + 1-D TMA bulk copies (cp.async.bulk, sm_90+; no tensor map, no multicast).
 // ---------------------------------------------------------------------------------

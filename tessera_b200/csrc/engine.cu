@@ -736,7 +736,7 @@ private:
     V *sites_ = nullptr, *theta_ = nullptr, *W_ = nullptr, *envs_ = nullptr, *xs_ = nullptr, *vbuf_ = nullptr;
     void* lqc_ = nullptr;  // cooperative LQ candidate rows
     bool lq_ok_ = false;
-    int *dims_ = nullptr, *perm_ = nullptr, *counters_ = nullptr, *step_ = nullptr;
+    int *dims_ = nullptr, *perm_ = nullptr, *counters_ = nullptr, *step_ = nullptr, *flags_ = nullptr;
     double* scal_ = nullptr;
     double *sig2_ = nullptr, *sig_ = nullptr, *h_ = nullptr, *w_ = nullptr, *sa_ = nullptr, *sb_ = nullptr;
     double *bias_ = nullptr, *sc_ = nullptr;
@@ -765,7 +765,7 @@ private:
     ScheduleView schedule() const {
         return ScheduleView{h_, w_, sa_, sb_, step_, C_.dt, C_.dt / C_.ns, bias_, sc_};
     }
-    SvdWork<T> work() const { return SvdWork<T>{theta_, W_, ld_, sig2_, sig_, perm_, counters_, scal_, bar_, stats_}; }
+    SvdWork<T> work() const { return SvdWork<T>{theta_, W_, ld_, sig2_, sig_, perm_, counters_, scal_, bar_, stats_, flags_}; }
 
     double tol_for(int R) const {
         if (C_.tol > 0) return C_.tol;
@@ -780,11 +780,11 @@ private:
     int pick_block(int R, int N) const {
         int b = std::min(C_.block, 16);  // a single instance has no block-Gram path
         if (!b) {
-            // default schedule: wide blocks for small matrices (few grid barriers), narrower
-            // ones for large matrices (enough block pairs to fill the SMs)
+            // wide blocks for small matrices (few rounds), narrower ones for large matrices (more
+            // block pairs, so more SMs).  complex128: 4, 64 CTAs at 512 columns, 11.2 ms a theta
+            // against 11.9 with 8 (320 columns: 6.1 against 6.7; 200: 7.1 against 7.0)
             if (N <= 64) b = 16;
-            else if (N <= 256) b = 8;
-            else b = 8;
+            else b = sizeof(T) == 8 ? 4 : 8;
         }
         const int rows_cap = (R + 7) & ~7;
         while (b > 1 && (size_t)2 * b * rows_cap * sizeof(V) > 200 * 1024) b >>= 1;
@@ -833,6 +833,7 @@ private:
         add((void**)&perm_, sizeof(int) * ld_);
         add((void**)&counters_, sizeof(int) * C_.max_sweeps);
         add((void**)&scal_, sizeof(double) * 2);
+        add((void**)&flags_, sizeof(int) * svd_flag_count(ld_));
         add((void**)&bar_, sizeof(GridBar));
         add((void**)&stats_, sizeof(RunStats));
         add((void**)&h_, sizeof(double) * n_);
@@ -853,8 +854,8 @@ private:
         add((void**)&dotout_, sizeof(double) * (1 + n_ + m_));
         add((void**)&amp2_, sizeof(double));
         add((void**)&spins_d_, n_);
-        // candidate rows of the cooperative LQ (theta of 257..1024 rows): 8 rows per CTA
-        lq_ok_ = ld_ > 256 && ld_ <= 1024;
+        // candidate rows of the cooperative LQ (theta up to 1024 rows that is not resident): 8 rows per CTA
+        lq_ok_ = ld_ > (sizeof(T) == 8 ? 64 : 256) && ld_ <= 1024;
         add((void**)&lqc_, lq_ok_ ? lq_coop_scratch_bytes(ld_, (int)es, (ld_ + 7) / 8) : 8);
         TQ_CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
         TQ_CK(device_alloc((void**)&base_, off));
@@ -951,10 +952,12 @@ private:
             }
         }
         if (!tc_done) launch_theta<T>(M, sch, op, nullptr, work(), dl, dr, stream_);
-        // theta above 256 rows (the cooperative column-pair Jacobi): the pivoted LQ first, unless
-        // switched off or a block width was forced
-        const bool lq = lq_ok_ && C_.precond != 2 && C_.block == 0 && 2 * dl > 256 && 2 * dl <= 1024 &&
-                        2 * dr <= 1024;
+        // the cooperative column-pair Jacobi: the pivoted LQ first, unless switched off or a block
+        // width was forced.  complex64: theta above 256 rows; complex128: every theta that is not
+        // resident in shared memory (200 x 200: 23 -> 10 sweeps, 7.1 -> 4.7 ms an update with the LQ;
+        // 128 x 128: 3.1 -> 2.7 ms)
+        const bool wide = sizeof(T) == 8 ? !svd_resident<T>(2 * dl, 2 * dr) : 2 * dl > 256;
+        const bool lq = lq_ok_ && C_.precond != 2 && C_.block == 0 && wide && 2 * dl <= 1024 && 2 * dr <= 1024;
         cudaEvent_t a = nullptr, b = nullptr;
         if (lq) {
             cudaEvent_t c = nullptr, d = nullptr;

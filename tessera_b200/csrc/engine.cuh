@@ -74,7 +74,11 @@ struct SvdWork {
     double* scal;       // [2] scratch scalars (squared Frobenius norm of W), zeroed per launch
     GridBar* bar;
     RunStats* stats;
+    int* flags;         // rounds each column block has been through (cooperative Jacobi) [svd_flag_count(ld)],
+                        // zeroed per launch
 };
+// column blocks of the cooperative Jacobi: at least 2 columns each, one more to make them even
+inline int svd_flag_count(int ld) { return (ld + 1) / 2 + 2; }
 
 struct SvdParams {
     int bond;
@@ -130,6 +134,9 @@ void launch_theta(const MpsView<T>& mps, const ScheduleView& sch, GateOp op, con
 template <typename T>
 int launch_svd(const MpsView<T>& mps, int bond, int chi, double tol, int max_sweeps, SvdWork<T> wk,
                int rows_ub, int cols_ub, int block_w, cudaStream_t s, int R = 0, int N = 0, int lq = 0, int rr = 0);
+// whether launch_svd keeps a theta of at most this size in one CTA's shared memory
+template <typename T>
+bool svd_resident(int rows_ub, int cols_ub);
 // cooperative row-pivoted LQ of one theta's working copy, in place (lq.cu); rows_ub <= 1024
 template <typename T>
 void launch_lq_coop(const MpsView<T>& mps, int bond, SvdWork<T> wk, void* scratch, int rows_ub, int cols_ub,

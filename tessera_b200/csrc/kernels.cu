@@ -577,8 +577,93 @@ __device__ void svd_finish(const MpsView<T>& mps, const SvdWork<T>& wk, const Sv
     }
 }
 
-// Whole SVD of one theta by `ncta` cooperating CTAs (this one is number `cta`); with
-// ncta == 1 a single CTA runs every block pair itself and needs no grid barrier.
+template <int RPL>
+__device__ __forceinline__ void lane_dot(const double2 (&x)[RPL], const double2 (&y)[RPL], double& re, double& im) {
+    double r0 = 0.0, r1 = 0.0, i0 = 0.0, i1 = 0.0;  // four chains
+#pragma unroll
+    for (int k = 0; k < RPL; ++k) {
+        r0 = fma(x[k].x, y[k].x, r0);
+        r1 = fma(x[k].y, y[k].y, r1);
+        i0 = fma(x[k].x, y[k].y, i0);
+        i1 = fma(-x[k].y, y[k].x, i1);
+    }
+    re = r0 + r1;
+    im = i0 + i1;
+}
+
+// sums of four doubles over the warp, to every lane: lanes hand over what they do not keep (two
+// values, then one), three levels on the one kept, and four broadcasts: 10 shuffles, not 20
+__device__ __forceinline__ void warp_sum4(double& a, double& b, double& c, double& d) {
+    const int lane = threadIdx.x & 31;
+    const bool h16 = lane & 16, h8 = lane & 8;
+    const double s0 = __shfl_xor_sync(0xffffffffu, h16 ? a : c, 16);
+    const double s1 = __shfl_xor_sync(0xffffffffu, h16 ? b : d, 16);
+    const double p = (h16 ? c : a) + s0, q = (h16 ? d : b) + s1;
+    double v = (h8 ? q : p) + __shfl_xor_sync(0xffffffffu, h8 ? p : q, 8);
+#pragma unroll
+    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    a = __shfl_sync(0xffffffffu, v, 0);
+    b = __shfl_sync(0xffffffffu, v, 8);
+    c = __shfl_sync(0xffffffffu, v, 16);
+    d = __shfl_sync(0xffffffffu, v, 24);
+}
+
+__device__ __forceinline__ void warp_sum2(double& a, double& b) {
+    const int lane = threadIdx.x & 31;
+    const bool h16 = lane & 16;
+    double v = (h16 ? b : a) + __shfl_xor_sync(0xffffffffu, h16 ? a : b, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+    a = __shfl_sync(0xffffffffu, v, 0);
+    b = __shfl_sync(0xffffffffu, v, 16);
+}
+
+// One pair of shared-memory columns p, q by one warp, with carried norms: 1 if rotated (lane 0).
+template <int RPL>
+__device__ __forceinline__ int pair_tracked(double2* col, const int rc, const int p, const int q, const int R,
+                                            const double tol, const double tiny, const bool mixed, double* nrm,
+                                            int* chg) {
+    const int lane = threadIdx.x & 31;
+    double2 x[RPL], y[RPL];
+#pragma unroll
+    for (int k = 0; k < RPL; ++k) {
+        const int row = lane + 32 * k;
+        x[k] = row < R ? col[p * rc + row] : make_double2(0.0, 0.0);
+        y[k] = row < R ? col[q * rc + row] : make_double2(0.0, 0.0);
+    }
+    double gr, gi, tr, ti;
+    const double a = nrm[p], b = nrm[q];
+    lane_dot<RPL>(x, y, gr, gi);
+    warp_sum2(gr, gi);
+    if (!jacobi_tau(a, b, gr, gi, tol * tol, tiny, mixed, tr, ti)) return 0;
+    const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2), cr = c * tr, ci = c * ti;
+#pragma unroll
+    for (int k = 0; k < RPL; ++k) {
+        const int row = lane + 32 * k;
+        if (row < R) {
+            const double2 u = x[k], v = y[k];
+            col[p * rc + row] = make_double2(fma(-ci, v.y, fma(-cr, v.x, c * u.x)), fma(ci, v.x, fma(-cr, v.y, c * u.y)));
+            col[q * rc + row] = make_double2(fma(-ci, u.y, fma(cr, u.x, c * v.x)), fma(ci, u.x, fma(cr, u.y, c * v.y)));
+        }
+    }
+    if (lane == 0) {
+        const double g = fma(tr, gr, ti * gi), c2 = c * c;
+        nrm[p] = fmax(0.0, c2 * fma(t2, b, fma(-2.0, g, a)));
+        nrm[q] = fmax(0.0, c2 * fma(t2, a, fma(2.0, g, b)));
+        chg[p] = 1;
+        chg[q] = 1;
+    }
+    return lane == 0 ? 1 : 0;
+}
+
+// Whole SVD of one theta by `ncta` cooperating CTAs (this one is number `cta`).  A CTA takes its next
+// block pair as soon as the two blocks' previous holders have released them (wk.flags, one counter
+// per block); the whole grid meets only at the end of a sweep.  Changed columns go back by bulk
+// copies.  complex128 carries norms and takes angles as svd_body_rcd does.  512 x 512 complex128
+// after the LQ, 11 sweeps: 12.6 ms with a grid barrier a round, 32 CTAs and element-wise stores,
+// 11.2 ms now; complex64 400 x 400: 7.3 -> 5.9 ms.  Bound: a round's chain on 64 of 148 SMs (stage
+// 64 KB, four dependent visits, store, flag); the pair arithmetic alone made no difference (13.5 ms
+// with 32 CTAs and the barrier).
 template <typename T, int BW, int RPL>
 __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>& wk, const SvdParams& pp,
                                          const int cta, const int ncta, unsigned char* smraw) {
@@ -590,6 +675,11 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
     __shared__ double red[4 * NW];         // [warps][4]
     __shared__ int s_rot;
     __shared__ __align__(8) uint64_t s_mbar;
+    // complex128 in registers (D): squared norms of the staged columns, summed at the start of a sweep
+    // (wk.sig2) and carried through each rotation, and which of the columns changed
+    constexpr bool D = sizeof(T) == 8 && RPL > 0;
+    __shared__ double s_n[2 * BW];
+    __shared__ int s_c[2 * BW];
     unsigned phase = 0;
     if (threadIdx.x == 0) mbar_init(&s_mbar, 1);
     __syncthreads();
@@ -646,6 +736,17 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
     bool converged = false;
     bool mixed = true;
     for (; sweep < pp.max_sweeps; ++sweep) {
+        if constexpr (D) {
+            const int warp = tid >> 5, lane = tid & 31;
+            for (int j = cta * NW + warp; j < N; j += ncta * NW) {
+                double sj = 0.0;
+                const V* w = W + (long long)j * ld;
+                for (int row = lane; row < R; row += 32) sj = fma(w[row].x, w[row].x, fma(w[row].y, w[row].y, sj));
+                sj = warp_sum(sj);
+                if (lane == 0) wk.sig2[j] = sj;
+            }
+            if (!cta_sync(wk.bar, status, nblk)) return;
+        }
         for (int r = 0; r < P - 1; ++r) {
             for (int pr = cta; pr < P / 2; pr += ncta) {
                 int I, J;
@@ -653,6 +754,13 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                 // stage columns with 1-D TMA bulk copies: local c < BW -> block I, c >= BW -> block J
                 if (tid == 0) {
                     s_rot = 0;
+                    // the two blocks as their previous holders left them (the others then time out on
+                    // the copy below and leave too)
+                    const int ver = sweep * (P - 1) + r;
+                    if (!flag_wait(&wk.flags[I], ver) || !flag_wait(&wk.flags[J], ver)) {
+                        atomicOr(status, ST_BARRIER_TIMEOUT);
+                        return;
+                    }
                     unsigned bytes = 0;
                     for (int c = 0; c < 2 * BW; ++c) {
                         const int gc = (c < BW) ? I * BW + c : J * BW + (c - BW);
@@ -675,7 +783,29 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                 }
                 phase ^= 1u;
                 int rot = 0;
-                if constexpr (BW >= 2) if (r == 0) {
+                if constexpr (D) {
+                    if (tid < 2 * BW) {
+                        const int gc = (tid < BW) ? I * BW + tid : J * BW + (tid - BW);
+                        s_n[tid] = gc < N ? __ldcg(&wk.sig2[gc]) : 0.0;  // (other CTAs wrote it)
+                        s_c[tid] = 0;
+                    }
+                    __syncthreads();
+                    if (r == 0) {  // pairs inside each block, one warp per pair
+                        const int half = BW / 2;
+                        const int blk = grp < half ? 0 : 1;
+                        const int ip = grp < half ? grp : grp - half;
+                        const int base = blk ? J * BW : I * BW;
+                        for (int t = 0; t < BW - 1; ++t) {
+                            int x, y;
+                            if (ip == 0) { x = BW - 1; y = t; }
+                            else { x = (t + ip) % (BW - 1); y = (t - ip + (BW - 1)) % (BW - 1); }
+                            if (base + x < N && base + y < N)
+                                rot += pair_tracked<RPL>(col, pp.rows_cap, blk * BW + x, blk * BW + y, R, pp.tol, tiny,
+                                                         mixed, s_n, s_c);
+                            __syncthreads();
+                        }
+                    }
+                } else if constexpr (BW >= 2) if (r == 0) {
                     // intra-block pairs: circle method over BW columns, both blocks at once
                     const int half = BW / 2;
                     const int blk = grp < half ? 0 : 1;
@@ -710,6 +840,7 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                         const int row = lane + 32 * k;
                         xi[k] = (row < R) ? ci[row] : czero<V>();
                     }
+                    double xn = D ? s_n[grp] : 0.0;
                     for (int t = 0; t < BW; ++t) {
                         const int q = (grp + t) % BW;
                         const bool ok = vi && (J * BW + q < N);
@@ -720,40 +851,58 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                             const int row = lane + 32 * k;
                             yj[k] = (row < R) ? cq[row] : czero<V>();
                         }
-                        double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
-                        if constexpr (sizeof(T) == 4) {
+                        if constexpr (D) {
+                            double gr, gi, tr, ti;
+                            const double a = xn, b = *(volatile double*)&s_n[BW + q];
+                            lane_dot<RPL>(xi, yj, gr, gi);
+                            warp_sum2(gr, gi);
+                            if (ok && jacobi_tau(a, b, gr, gi, pp.tol * pp.tol, tiny, mixed, tr, ti)) {
+                                const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2);
+                                const double cr = c * tr, cim = c * ti;
+#pragma unroll
+                                for (int k = 0; k < RPL; ++k) {
+                                    const int row = lane + 32 * k;
+                                    const V u = xi[k], v = yj[k];
+                                    xi[k].x = fma(-cim, v.y, fma(-cr, v.x, c * u.x));
+                                    xi[k].y = fma(cim, v.x, fma(-cr, v.y, c * u.y));
+                                    const V z = make_double2(fma(-cim, u.y, fma(cr, u.x, c * v.x)),
+                                                             fma(cim, u.x, fma(cr, u.y, c * v.y)));
+                                    if (row < R) cq[row] = z;
+                                }
+                                const double g = fma(tr, gr, ti * gi), c2 = c * c;
+                                xn = fmax(0.0, c2 * fma(t2, b, fma(-2.0, g, a)));
+                                if (lane == 0) {
+                                    s_n[BW + q] = fmax(0.0, c2 * fma(t2, a, fma(2.0, g, b)));
+                                    s_c[BW + q] = 1;
+                                    s_c[grp] = 1;
+                                    ++rot;
+                                }
+                            }
+                        } else {
+                            double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
                             LaneDotsF32 d;
 #pragma unroll
                             for (int k = 0; k < RPL; ++k) d.add(xi[k], yj[k]);
                             v0 = d.a; v1 = d.b; v2 = d.gr; v3 = d.gi;
-                        } else {
 #pragma unroll
-                            for (int k = 0; k < RPL; ++k) {
-                                const V x = xi[k], y = yj[k];
-                                v0 += (double)x.x * x.x + (double)x.y * x.y;
-                                v1 += (double)y.x * y.x + (double)y.y * y.y;
-                                v2 += (double)x.x * y.x + (double)x.y * y.y;
-                                v3 += (double)x.x * y.y - (double)x.y * y.x;
+                            for (int o = 16; o > 0; o >>= 1) {
+                                v0 += __shfl_xor_sync(0xffffffffu, v0, o);
+                                v1 += __shfl_xor_sync(0xffffffffu, v1, o);
+                                v2 += __shfl_xor_sync(0xffffffffu, v2, o);
+                                v3 += __shfl_xor_sync(0xffffffffu, v3, o);
                             }
-                        }
+                            T c, sn, er, ei;
+                            if (ok && jacobi_rotation<T>(v0, v1, v2, v3, pp.tol, tiny, mixed, c, sn, er, ei)) {
+                                const PairRot<T> rt(c, sn, er, ei);
 #pragma unroll
-                        for (int o = 16; o > 0; o >>= 1) {
-                            v0 += __shfl_xor_sync(0xffffffffu, v0, o);
-                            v1 += __shfl_xor_sync(0xffffffffu, v1, o);
-                            v2 += __shfl_xor_sync(0xffffffffu, v2, o);
-                            v3 += __shfl_xor_sync(0xffffffffu, v3, o);
-                        }
-                        T c, sn, er, ei;
-                        if (ok && jacobi_rotation<T>(v0, v1, v2, v3, pp.tol, tiny, mixed, c, sn, er, ei)) {
-                            const PairRot<T> rt(c, sn, er, ei);
+                                for (int k = 0; k < RPL; ++k) rt.apply(xi[k], yj[k]);
 #pragma unroll
-                            for (int k = 0; k < RPL; ++k) rt.apply(xi[k], yj[k]);
-#pragma unroll
-                            for (int k = 0; k < RPL; ++k) {
-                                const int row = lane + 32 * k;
-                                if (row < R) cq[row] = yj[k];
+                                for (int k = 0; k < RPL; ++k) {
+                                    const int row = lane + 32 * k;
+                                    if (row < R) cq[row] = yj[k];
+                                }
+                                if (lane == 0) ++rot;
                             }
-                            if (lane == 0) ++rot;
                         }
                         __syncthreads();
                     }
@@ -762,22 +911,37 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                         const int row = lane + 32 * k;
                         if (row < R) ci[row] = xi[k];
                     }
+                    if (D && lane == 0) s_n[grp] = xn;
                     __syncthreads();
                 }
                 if (rot && (tid % G) == 0) atomicAdd(&s_rot, rot);
-                __syncthreads();
-                for (int c = 0; c < 2 * BW; ++c) {
-                    const int gc = (c < BW) ? I * BW + c : J * BW + (c - BW);
-                    if (gc >= N) continue;
-                    V* dst = W + (long long)gc * ld;
-                    const V* src = col + c * pp.rows_cap;
-                    for (int row = tid; row < R; row += NT) dst[row] = src[row];
+                if (D && tid < 2 * BW && s_c[tid]) {
+                    const int gc = (tid < BW) ? I * BW + tid : J * BW + (tid - BW);
+                    wk.sig2[gc] = s_n[tid];
                 }
-                if (tid == 0 && s_rot) atomicAdd(&wk.counters[sweep], s_rot);
+                fence_proxy_async_shared();  // the bulk copies below read what these threads wrote
+                __syncthreads();
+                if (tid == 0) {
+                    // the columns (complex128: those that changed) back by bulk copies, then the blocks
+                    // go to their next holders
+                    for (int c = 0; c < 2 * BW; ++c) {
+                        const int gc = (c < BW) ? I * BW + c : J * BW + (c - BW);
+                        if (gc >= N || (D ? !s_c[c] : !s_rot)) continue;
+                        tma_store_1d(W + (long long)gc * ld, col + c * pp.rows_cap, (unsigned)(R * sizeof(V)));
+                    }
+                    tma_store_commit();
+                    if (s_rot) atomicAdd(&wk.counters[sweep], s_rot);
+                    tma_store_wait_all();
+                    fence_proxy_async_global();
+                    __threadfence();
+                    const int ver = sweep * (P - 1) + r + 1;
+                    flag_release(&wk.flags[I], ver);
+                    flag_release(&wk.flags[J], ver);
+                }
                 __syncthreads();
             }
-            if (!cta_sync(wk.bar, status, nblk)) return;
         }
+        if (!cta_sync(wk.bar, status, nblk)) return;
         const int done = *(volatile int*)&wk.counters[sweep];
         if (done == 0) {
             converged = true;
@@ -2289,47 +2453,6 @@ struct RotCoef {
     }
 };
 
-template <int RPL>
-__device__ __forceinline__ void lane_dot(const double2 (&x)[RPL], const double2 (&y)[RPL], double& re, double& im) {
-    double r0 = 0.0, r1 = 0.0, i0 = 0.0, i1 = 0.0;  // four chains
-#pragma unroll
-    for (int k = 0; k < RPL; ++k) {
-        r0 = fma(x[k].x, y[k].x, r0);
-        r1 = fma(x[k].y, y[k].y, r1);
-        i0 = fma(x[k].x, y[k].y, i0);
-        i1 = fma(-x[k].y, y[k].x, i1);
-    }
-    re = r0 + r1;
-    im = i0 + i1;
-}
-
-// sums of four doubles over the warp, to every lane: lanes hand over what they do not keep (two
-// values, then one), three levels on the one kept, and four broadcasts: 10 shuffles, not 20
-__device__ __forceinline__ void warp_sum4(double& a, double& b, double& c, double& d) {
-    const int lane = threadIdx.x & 31;
-    const bool h16 = lane & 16, h8 = lane & 8;
-    const double s0 = __shfl_xor_sync(0xffffffffu, h16 ? a : c, 16);
-    const double s1 = __shfl_xor_sync(0xffffffffu, h16 ? b : d, 16);
-    const double p = (h16 ? c : a) + s0, q = (h16 ? d : b) + s1;
-    double v = (h8 ? q : p) + __shfl_xor_sync(0xffffffffu, h8 ? p : q, 8);
-#pragma unroll
-    for (int o = 4; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    a = __shfl_sync(0xffffffffu, v, 0);
-    b = __shfl_sync(0xffffffffu, v, 8);
-    c = __shfl_sync(0xffffffffu, v, 16);
-    d = __shfl_sync(0xffffffffu, v, 24);
-}
-
-__device__ __forceinline__ void warp_sum2(double& a, double& b) {
-    const int lane = threadIdx.x & 31;
-    const bool h16 = lane & 16;
-    double v = (h16 ? b : a) + __shfl_xor_sync(0xffffffffu, h16 ? a : b, 16);
-#pragma unroll
-    for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-    a = __shfl_sync(0xffffffffu, v, 0);
-    b = __shfl_sync(0xffffffffu, v, 16);
-}
-
 template <int NW, int RPL>
 __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& wk, const SvdParams& pp,
                              unsigned char* smraw) {
@@ -2789,6 +2912,21 @@ static int svd_launch_bw(const MpsView<T>& mps, const SvdParams& pp, SvdWork<T> 
     return grid;
 }
 
+// shared-memory column length and count for theta's upper bounds
+static void svd_caps(int rows_ub, int cols_ub, int& rows_cap, int& cols_cap) {
+    rows_cap = (rows_ub + 7) & ~7;
+    if (rows_cap < 8) rows_cap = 8;
+    cols_cap = (cols_ub + 1) & ~1;
+    if (cols_cap < 2) cols_cap = 2;
+}
+
+template <typename T>
+bool svd_resident(int rows_ub, int cols_ub) {
+    int r, c;
+    svd_caps(rows_ub, cols_ub, r, c);
+    return resident_smem<T>(r, c) != 0;
+}
+
 template <typename T>
 int launch_svd(const MpsView<T>& mps, int bond, int chi, double tol, int max_sweeps, SvdWork<T> wk,
                int rows_ub, int cols_ub, int block_w, cudaStream_t s, int R, int N, int lq, int rr) {
@@ -2803,14 +2941,12 @@ int launch_svd(const MpsView<T>& mps, int bond, int chi, double tol, int max_swe
     pp.tol = tol;
     pp.tiny = sizeof(T) == 8 ? 1e-200 : 1e-60;
     pp.max_sweeps = max_sweeps;
-    pp.rows_cap = (rows_ub + 7) & ~7;
-    if (pp.rows_cap < 8) pp.rows_cap = 8;
-    pp.cols_cap = (cols_ub + 1) & ~1;
-    if (pp.cols_cap < 2) pp.cols_cap = 2;
+    svd_caps(rows_ub, cols_ub, pp.rows_cap, pp.cols_cap);
     // small theta: the whole matrix stays in one CTA's shared memory
     if (res_dispatch<T>(&mps, &wk, pp, nullptr, nullptr, 0, s)) return 1;
     TQ_CHECK(cudaMemsetAsync(wk.counters, 0, sizeof(int) * max_sweeps, s));
     TQ_CHECK(cudaMemsetAsync(wk.scal, 0, sizeof(double) * 2, s));
+    TQ_CHECK(cudaMemsetAsync(wk.flags, 0, sizeof(int) * svd_flag_count(wk.ld), s));
     // register-resident path for rows <= 512: rows per lane = next power of two >= rows/32
     int rpl = 1;
     while (32 * rpl < pp.rows_cap) rpl <<= 1;
@@ -3433,9 +3569,11 @@ int launch_update_batch(const InstTask<T>* insts, const UpdRef* refs, int nref, 
     // 32 is asked for
     if (block_w == 0) bw = (sizeof(T) == 4 && rpl == 16) ? 16 : 8;
     if (sizeof(T) == 8 && bw > 8) bw = 8;  // two columns a warp: 16 warps leave too few registers
-    // the pivoted LQ preconditioner for the column-pair kernel at 257..512 rows (outside the
-    // svd_begin/svd_end window, so that window times the Jacobi alone)
-    const int lq = (precond && block_w != BG_B && rpl == 16 && resident_smem<T>(rows_cap, rows_cap) == 0) ? 1 : 0;
+    // the pivoted LQ preconditioner for the column-pair kernel (outside the svd_begin/svd_end window,
+    // so that window times the Jacobi alone): complex64 at 257..512 rows, complex128 wherever theta
+    // is not resident
+    const int lq = (precond && block_w != BG_B && (sizeof(T) == 8 || rpl == 16) &&
+                    resident_smem<T>(rows_cap, rows_cap) == 0) ? 1 : 0;
     if (lq) {  // lq_begin/lq_end are recorded only here: a return of 5 launches says they were
         if (lq_begin) TQ_CHECK(cudaEventRecord(lq_begin, s));
         launch_lq_batch<T>(insts, refs, nref, s);
@@ -3493,6 +3631,7 @@ void launch_entropy_batch(const InstTask<T>* insts, int ninst, cudaStream_t s) {
     template void launch_single_site<T>(const MpsView<T>&, const ScheduleView&, int, cudaStream_t);         \
     template void launch_theta<T>(const MpsView<T>&, const ScheduleView&, GateOp, const double*, SvdWork<T>, \
                                   int, int, cudaStream_t);                                                  \
+    template bool svd_resident<T>(int, int);                                                                \
     template int launch_svd<T>(const MpsView<T>&, int, int, double, int, SvdWork<T>, int, int, int,         \
                                cudaStream_t, int, int, int, int);                                           \
     template void launch_absorb<T>(const MpsView<T>&, int, SvdWork<T>, int, int, int, cudaStream_t);        \

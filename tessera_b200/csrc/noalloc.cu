@@ -36,6 +36,7 @@ struct NoAllocScratch {
     int perm[kNoAllocMaxDim];
     int counters[kNoAllocSweeps];
     double scal[2];
+    int flags[kNoAllocMaxDim / 2 + 3];
     GridBar bar;
     RunStats stats;
 };
@@ -116,7 +117,7 @@ extern "C" int tessera_qa_svd_noalloc(const double* d_a, size_t rows, size_t col
             e = cudaGetLastError();
             if (e != cudaSuccess) throw std::runtime_error(std::string("launch: ") + cudaGetErrorString(e));
             SvdWork<double> wk{nullptr, sc->W, kNoAllocMaxDim, sc->sig2, sc->sig, sc->perm,
-                               sc->counters, sc->scal, &sc->bar, &sc->stats};
+                               sc->counters, sc->scal, &sc->bar, &sc->stats, sc->flags};
             MpsView<double> none{nullptr, nullptr, 0, 1, 0};
             const int bw = N <= 64 ? 16 : 8;
             const double tol = 1e-13;
