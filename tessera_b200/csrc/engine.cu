@@ -53,8 +53,9 @@ static int g_fail_after = 0, g_fail_count = 0;
 // The library's own memory pool on each device.  cudaMalloc and cudaFree map and unmap pages and
 // wait for the whole device: on one box 0.1 ms a pair, on another 3 ms, and more for 100 MB, beside
 // kernels of a few microseconds; a call that makes an engine, runs it and drops it paid that several
-// times.  Freed memory stays in the pool up to kKeep bytes per device; what is above goes back to
-// the driver at each free, all of it when an allocation fails or device_trim() is called, and the
+// times.  The pool holds at most kKeep bytes per device; an allocation that would take it further is
+// a plain cudaMalloc (148 arenas of 55 MB: 0.13 s through the pool, 0.09 s that way).  What the pool
+// holds unused goes back to the driver when an allocation fails or device_trim() is called, and the
 // pools end with the process.  Allocation and release run on a stream of the pool's own that no
 // kernel uses, and are waited for, so the memory is good for any stream and thread when alloc()
 // returns; callers have waited for their work before they free, as cudaFree's callers had not to.
@@ -70,26 +71,35 @@ public:
         if (e != cudaSuccess) return e;
         std::lock_guard<std::mutex> lk(mu_);
         Pool* pl = pool(dev);
-        if (!pl) return cudaMalloc(out, bytes);
+        const bool pooled = pl && pl->used + bytes <= kKeep;
         for (int turn = 0; turn < 2; ++turn) {
-            e = cudaMallocFromPoolAsync(out, bytes, pl->pool, pl->st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(pl->st);
-            if (e != cudaErrorMemoryAllocation) break;
+            if (pooled) {
+                e = cudaMallocFromPoolAsync(out, bytes, pl->pool, pl->st);
+                if (e == cudaSuccess) e = cudaStreamSynchronize(pl->st);
+            } else {
+                e = cudaMalloc(out, bytes);
+            }
+            if (e != cudaErrorMemoryAllocation || !pl) break;
             cudaGetLastError();  // not sticky: the caller reports it, or the second turn succeeds
             if (turn == 0) cudaMemPoolTrimTo(pl->pool, 0);
         }
-        if (e == cudaSuccess) owner_[*out] = dev;
+        if (e == cudaSuccess && pooled) {
+            owner_[*out] = Block{dev, bytes};
+            pl->used += bytes;
+        }
         return e;
     }
     void free(void* p) {
         if (!p) return;
-        std::lock_guard<std::mutex> lk(mu_);
+        std::unique_lock<std::mutex> lk(mu_);
         auto it = owner_.find(p);
         if (it == owner_.end()) {
+            lk.unlock();
             cudaFree(p);
             return;
         }
-        Pool& pl = pools_[it->second];
+        Pool& pl = pools_[it->second.dev];
+        pl.used -= it->second.bytes;
         owner_.erase(it);
         cudaFreeAsync(p, pl.st);
         cudaStreamSynchronize(pl.st);
@@ -107,6 +117,11 @@ private:
         int state = 0;  // 0 not tried, 1 ready, 2 not to be had on this device
         cudaMemPool_t pool = nullptr;
         cudaStream_t st = nullptr;
+        size_t used = 0;  // bytes handed out
+    };
+    struct Block {
+        int dev;
+        size_t bytes;
     };
     Pool* pool(int dev) {  // dev is current; nullptr: plain cudaMalloc
         if (dev < 0 || dev >= kMax) return nullptr;
@@ -132,7 +147,7 @@ private:
     }
     std::mutex mu_;
     Pool pools_[kMax];
-    std::unordered_map<void*, int> owner_;
+    std::unordered_map<void*, Block> owner_;
 };
 
 cudaError_t device_alloc(void** p, size_t bytes) {
