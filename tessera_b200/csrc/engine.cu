@@ -320,6 +320,52 @@ public:
 static const char kMagic[8] = {'T', 'Q', 'M', 'P', 'S', 'v', '1', 0};
 static size_t ckpt_header_bytes(int n) { return 32 + ((size_t)4 * (n + 1) + 7) / 8 * 8; }
 
+// Standalone SVD output: the U columns whose singular value lies under the Jacobi's noise floor
+// (8 sqrt(R) ulps of ||A||_F) carry rounding noise, not a resolved direction.  Each is replaced,
+// in descending order, by its part orthogonal to every column before it (classical Gram-Schmidt,
+// two passes), renormalised; a column with nothing left becomes zero.  U (R x k, row-major) is
+// then an isometry on its non-zero columns, as the reference's SVD makes its factor by
+// Gram-Schmidt (cuda/src/linalg.cpp:56-105).
+static double noise_floor(int R, const std::vector<double>& sig) {
+    double fro2 = 0.0;
+    for (double x : sig) fro2 += x * x;
+    return 8.0 * std::sqrt((double)R) * 2.220446049250313e-16 * std::sqrt(fro2);
+}
+static bool has_subfloor(int R, const std::vector<double>& sig) {
+    const double floor = noise_floor(R, sig);
+    for (double x : sig)
+        if (!(x > floor)) return true;
+    return false;
+}
+static void orthonormalise_subfloor(std::vector<double2>& U, int R, int k, const std::vector<double>& sig) {
+    const double floor = noise_floor(R, sig);
+    std::vector<double2> x(R);
+    for (int t = 0; t < k; ++t) {
+        if (sig[t] > floor) continue;
+        for (int i = 0; i < R; ++i) x[i] = U[(size_t)i * k + t];
+        double n0 = 0.0;
+        for (int i = 0; i < R; ++i) n0 += x[i].x * x[i].x + x[i].y * x[i].y;
+        for (int pass = 0; pass < 2; ++pass)
+            for (int q = 0; q < t; ++q) {
+                double re = 0.0, im = 0.0;  // u_q^H x
+                for (int i = 0; i < R; ++i) {
+                    const double2 u = U[(size_t)i * k + q];
+                    re += u.x * x[i].x + u.y * x[i].y;
+                    im += u.x * x[i].y - u.y * x[i].x;
+                }
+                for (int i = 0; i < R; ++i) {
+                    const double2 u = U[(size_t)i * k + q];
+                    x[i].x -= re * u.x - im * u.y;
+                    x[i].y -= re * u.y + im * u.x;
+                }
+            }
+        double n2 = 0.0;
+        for (int i = 0; i < R; ++i) n2 += x[i].x * x[i].x + x[i].y * x[i].y;
+        const double sc = (n0 > 0.0 && n2 > 1e-16 * n0) ? 1.0 / std::sqrt(n2) : 0.0;
+        for (int i = 0; i < R; ++i) U[(size_t)i * k + t] = make_double2(x[i].x * sc, x[i].y * sc);
+    }
+}
+
 template <typename T>
 class Engine final : public EngineBase {
     using V = cplx_t<T>;
@@ -656,25 +702,52 @@ public:
         ub_ = d;
     }
 
-    // standalone SVD of an R x N matrix (column-major in W) -> perm, sig
-    void svd_only(const std::vector<V>& colmajor, int R, int N, std::vector<int>& perm, std::vector<double>& sig,
-                  std::vector<V>& Wout) {
-        TQ_CK(cudaMemcpy2DAsync(W_, ld_ * sizeof(V), colmajor.data(), R * sizeof(V), R * sizeof(V), N,
-                                cudaMemcpyHostToDevice, stream_));
-        const int bw = pick_block(R, N);
-        launch_svd<T>(mps(), 0, std::min(R, N), tol_for(R), C_.max_sweeps, work(), R, N, bw, stream_, R, N);
+    // Standalone thin SVD of a row-major R x N matrix: s (k = min(R, N)), u (R x k) and vh (k x N), each
+    // row-major, u and vh optional.  W takes a transposed copy, the factors are formed on the device:
+    // u from W's columns, vh = diag(1/s) u^H a as a tiled product.  Only when singular values lie under
+    // the Jacobi's noise floor does u visit the host, to have those columns completed.
+    void svd_only(const double2* a, int R, int N, double* s, double2* u, double2* vh) {
         const int k = std::min(R, N);
-        perm.resize(k);
-        sig.resize(k);
-        Wout.resize((size_t)R * N);
-        TQ_CK(cudaMemcpyAsync(perm.data(), perm_, sizeof(int) * k, cudaMemcpyDeviceToHost, stream_));
-        TQ_CK(cudaMemcpyAsync(sig.data(), sig_, sizeof(double) * k, cudaMemcpyDeviceToHost, stream_));
-        TQ_CK(cudaMemcpy2DAsync(Wout.data(), R * sizeof(V), W_, ld_ * sizeof(V), R * sizeof(V), N,
-                                cudaMemcpyDeviceToHost, stream_));
-        TQ_CK(cudaStreamSynchronize(stream_));
+        const size_t na = align256(sizeof(V) * (size_t)R * N), nu = align256(sizeof(V) * (size_t)R * k);
+        struct Buf {  // released on every way out
+            char* p = nullptr;
+            cudaStream_t st;
+            ~Buf() {
+                if (p) cudaStreamSynchronize(st);
+                device_free(p);
+            }
+        } buf;
+        buf.st = stream_;
+        TQ_CK(device_alloc((void**)&buf.p, na + nu + align256(sizeof(V) * (size_t)k * N)));
+        V* da = reinterpret_cast<V*>(buf.p);
+        V* du = reinterpret_cast<V*>(buf.p + na);
+        V* dv = reinterpret_cast<V*>(buf.p + na + nu);
+        TQ_CK(cudaMemcpyAsync(da, a, sizeof(V) * (size_t)R * N, cudaMemcpyHostToDevice, stream_));
+        launch_svd_load<T>(da, R, N, W_, ld_, stream_);
+        const int bw = pick_block(R, N);
+        launch_svd<T>(mps(), 0, k, tol_for(R), C_.max_sweeps, work(), R, N, bw, stream_, R, N);
+        if (u || vh) launch_svd_u<T>(W_, ld_, perm_, sig_, R, k, du, stream_);
+        std::vector<double> sg(k);
         RunStats st;
-        TQ_CK(cudaMemcpy(&st, stats_, sizeof(st), cudaMemcpyDeviceToHost));
+        TQ_CK(cudaMemcpyAsync(sg.data(), sig_, sizeof(double) * k, cudaMemcpyDeviceToHost, stream_));
+        TQ_CK(cudaMemcpyAsync(&st, stats_, sizeof(st), cudaMemcpyDeviceToHost, stream_));
+        TQ_CK(cudaStreamSynchronize(stream_));
         status_ = st.status;
+        std::vector<double2> U;
+        if ((u || vh) && has_subfloor(R, sg)) {
+            U.resize((size_t)R * k);
+            TQ_CK(cudaMemcpyAsync(U.data(), du, sizeof(V) * U.size(), cudaMemcpyDeviceToHost, stream_));
+            TQ_CK(cudaStreamSynchronize(stream_));
+            orthonormalise_subfloor(U, R, k, sg);
+            TQ_CK(cudaMemcpyAsync(du, U.data(), sizeof(V) * U.size(), cudaMemcpyHostToDevice, stream_));
+        }
+        if (vh) {
+            launch_svd_vh<T>(du, da, sig_, R, k, N, dv, stream_);
+            TQ_CK(cudaMemcpyAsync(vh, dv, sizeof(V) * (size_t)k * N, cudaMemcpyDeviceToHost, stream_));
+        }
+        if (u) TQ_CK(cudaMemcpyAsync(u, du, sizeof(V) * (size_t)R * k, cudaMemcpyDeviceToHost, stream_));
+        TQ_CK(cudaStreamSynchronize(stream_));
+        std::copy(sg.begin(), sg.end(), s);
     }
     int status_ = 0;
     int cap() const { return cap_; }
@@ -1443,43 +1516,6 @@ static void run_batch(const std::vector<ProblemHost>& P, const std::vector<Confi
     }
 }
 
-// Standalone SVD output: the U columns whose singular value lies under the Jacobi's noise floor
-// (8 sqrt(R) ulps of ||A||_F) carry rounding noise, not a resolved direction.  Each is replaced,
-// in descending order, by its part orthogonal to every column before it (classical Gram-Schmidt,
-// two passes), renormalised; a column with nothing left becomes zero.  U (R x k, row-major) is
-// then an isometry on its non-zero columns, as the reference's SVD makes its factor by
-// Gram-Schmidt (cuda/src/linalg.cpp:56-105).
-static void orthonormalise_subfloor(std::vector<double2>& U, int R, int k, const std::vector<double>& sig) {
-    double fro2 = 0.0;
-    for (int t = 0; t < k; ++t) fro2 += sig[t] * sig[t];
-    const double floor = 8.0 * std::sqrt((double)R) * 2.220446049250313e-16 * std::sqrt(fro2);
-    std::vector<double2> x(R);
-    for (int t = 0; t < k; ++t) {
-        if (sig[t] > floor) continue;
-        for (int i = 0; i < R; ++i) x[i] = U[(size_t)i * k + t];
-        double n0 = 0.0;
-        for (int i = 0; i < R; ++i) n0 += x[i].x * x[i].x + x[i].y * x[i].y;
-        for (int pass = 0; pass < 2; ++pass)
-            for (int q = 0; q < t; ++q) {
-                double re = 0.0, im = 0.0;  // u_q^H x
-                for (int i = 0; i < R; ++i) {
-                    const double2 u = U[(size_t)i * k + q];
-                    re += u.x * x[i].x + u.y * x[i].y;
-                    im += u.x * x[i].y - u.y * x[i].x;
-                }
-                for (int i = 0; i < R; ++i) {
-                    const double2 u = U[(size_t)i * k + q];
-                    x[i].x -= re * u.x - im * u.y;
-                    x[i].y -= re * u.y + im * u.x;
-                }
-            }
-        double n2 = 0.0;
-        for (int i = 0; i < R; ++i) n2 += x[i].x * x[i].x + x[i].y * x[i].y;
-        const double sc = (n0 > 0.0 && n2 > 1e-16 * n0) ? 1.0 / std::sqrt(n2) : 0.0;
-        for (int i = 0; i < R; ++i) U[(size_t)i * k + t] = make_double2(x[i].x * sc, x[i].y * sc);
-    }
-}
-
 }  // namespace tq
 
 using namespace tq;
@@ -1627,7 +1663,7 @@ int tessera_qa_svd(const double* a, size_t rows, size_t cols, double* s, double*
     return guarded([&]() -> int {
         if (!a || !s) throw ArgError("a or s is NULL");
         if (rows == 0 || cols == 0 || rows > 2048 || cols > 2048) throw ArgError("matrix shape out of range");
-        const int R = (int)rows, N = (int)cols, k = std::min(R, N);
+        const int R = (int)rows, N = (int)cols;
         ProblemHost P;
         P.n = 1;
         P.h.assign(1, 0.0);
@@ -1637,42 +1673,8 @@ int tessera_qa_svd(const double* a, size_t rows, size_t cols, double* s, double*
         int dev = 0;
         if (cudaGetDeviceCount(&dev) != cudaSuccess || dev == 0) throw CudaError("no CUDA device available");
         Engine<double> eng(P, C);
-        std::vector<double2> cm((size_t)R * N);
-        for (int i = 0; i < R; ++i)
-            for (int j = 0; j < N; ++j) cm[(size_t)j * R + i] = make_double2(a[2 * ((size_t)i * N + j)], a[2 * ((size_t)i * N + j) + 1]);
-        std::vector<int> perm;
-        std::vector<double> sig;
-        std::vector<double2> Wc;
-        eng.svd_only(cm, R, N, perm, sig, Wc);
-        for (int t = 0; t < k; ++t) s[t] = sig[t];
-        if (u || vh) {
-            // U[:, t] = W[:, perm[t]] / sigma_t ; Vh[t, :] = U[:, t]^H A
-            std::vector<double2> U((size_t)R * k, make_double2(0, 0));
-            for (int t = 0; t < k; ++t) {
-                if (!(sig[t] > 1e-300)) continue;
-                for (int i = 0; i < R; ++i) {
-                    const double2 w = Wc[(size_t)perm[t] * R + i];
-                    U[(size_t)i * k + t] = make_double2(w.x / sig[t], w.y / sig[t]);
-                }
-            }
-            orthonormalise_subfloor(U, R, k, sig);
-            if (u) std::memcpy(u, U.data(), sizeof(double2) * U.size());
-            if (vh) {
-                for (int t = 0; t < k; ++t)
-                    for (int j = 0; j < N; ++j) {
-                        double re = 0, im = 0;
-                        if (sig[t] > 1e-300)
-                            for (int i = 0; i < R; ++i) {
-                                const double2 x = U[(size_t)i * k + t];
-                                const double ar = a[2 * ((size_t)i * N + j)], ai = a[2 * ((size_t)i * N + j) + 1];
-                                re += x.x * ar + x.y * ai;
-                                im += x.x * ai - x.y * ar;
-                            }
-                        vh[2 * ((size_t)t * N + j)] = re / (sig[t] > 1e-300 ? sig[t] : 1.0);
-                        vh[2 * ((size_t)t * N + j) + 1] = im / (sig[t] > 1e-300 ? sig[t] : 1.0);
-                    }
-            }
-        }
+        eng.svd_only(reinterpret_cast<const double2*>(a), R, N, s, reinterpret_cast<double2*>(u),
+                     reinterpret_cast<double2*>(vh));
         if (eng.status_) {
             set_err("kernel status bits set: " + std::to_string(eng.status_));
             return TESSERA_QA_ESTATUS;

@@ -134,6 +134,16 @@ void launch_theta(const MpsView<T>& mps, const ScheduleView& sch, GateOp op, con
 template <typename T>
 int launch_svd(const MpsView<T>& mps, int bond, int chi, double tol, int max_sweeps, SvdWork<T> wk,
                int rows_ub, int cols_ub, int block_w, cudaStream_t s, int R = 0, int N = 0, int lq = 0, int rr = 0);
+// standalone SVD: row-major a into column-major W; u[i, t] = W[i, perm[t]] / s[t] (zero where s[t] is
+// at most 1e-300), row-major R x k; vh = diag(1/s) u^H a, row-major k x N, rows alike
+template <typename T>
+void launch_svd_load(const cplx_t<T>* a, int R, int N, cplx_t<T>* W, int ld, cudaStream_t s);
+template <typename T>
+void launch_svd_u(const cplx_t<T>* W, int ld, const int* perm, const double* sig, int R, int k, cplx_t<T>* u,
+                  cudaStream_t s);
+template <typename T>
+void launch_svd_vh(const cplx_t<T>* u, const cplx_t<T>* a, const double* sig, int R, int k, int N, cplx_t<T>* vh,
+                   cudaStream_t s);
 // whether launch_svd keeps a theta of at most this size in one CTA's shared memory
 template <typename T>
 bool svd_resident(int rows_ub, int cols_ub);

@@ -3097,6 +3097,73 @@ __device__ void gemm_phase(int M, int N, int K, LA la, LB lb, ST st, V (*As)[32]
     }
 }
 
+// ------------------------------------------------------------------------------------
+// Standalone SVD, around the Jacobi: the transposed load, U from W's columns, and Vh = diag(1/s) U^H A
+// as 32 x 32 tiles.  (Host loops before, a strided walk over U for every element of Vh: 55 of 69 ms at
+// 320 x 320.)
+// ------------------------------------------------------------------------------------
+template <typename T>
+__global__ void k_svd_load(const cplx_t<T>* a, int R, int N, cplx_t<T>* W, int ld) {
+    __shared__ cplx_t<T> tile[32][33];
+    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+        if (r0 + y < R && c0 + threadIdx.x < N) tile[y][threadIdx.x] = a[(long long)(r0 + y) * N + c0 + threadIdx.x];
+    __syncthreads();
+    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+        if (c0 + y < N && r0 + threadIdx.x < R) W[(long long)(c0 + y) * ld + r0 + threadIdx.x] = tile[threadIdx.x][y];
+}
+
+template <typename T>
+__global__ void k_svd_u(const cplx_t<T>* W, int ld, const int* perm, const double* sig, int R, int k, cplx_t<T>* u) {
+    using V = cplx_t<T>;
+    __shared__ V tile[32][33];
+    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
+    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+        if (c0 + y < k && r0 + threadIdx.x < R) {
+            const double sg = sig[c0 + y];
+            const V w = W[(long long)perm[c0 + y] * ld + r0 + threadIdx.x];
+            tile[threadIdx.x][y] = sg > 1e-300 ? mk<V>((T)(w.x / sg), (T)(w.y / sg)) : czero<V>();
+        }
+    __syncthreads();
+    for (int y = threadIdx.y; y < 32; y += blockDim.y)
+        if (r0 + y < R && c0 + threadIdx.x < k) u[(long long)(r0 + y) * k + c0 + threadIdx.x] = tile[y][threadIdx.x];
+}
+
+template <typename T>
+__global__ void __launch_bounds__(256) k_svd_vh(const cplx_t<T>* u, const cplx_t<T>* a, const double* sig, int R, int k,
+                                                int N, cplx_t<T>* vh) {
+    using V = cplx_t<T>;
+    __shared__ V As[8][32];
+    __shared__ V Bs[8][32];
+    gemm_phase<V>(k, N, R,
+        [&](int i, int r) { V v = u[(long long)r * k + i]; v.y = -v.y; return v; },
+        [&](int r, int j) { return a[(long long)r * N + j]; },
+        [&](int i, int j, V v) {
+            const double sg = sig[i];
+            vh[(long long)i * N + j] = sg > 1e-300 ? mk<V>((T)(v.x / sg), (T)(v.y / sg)) : czero<V>();
+        }, As, Bs, blockIdx.x, gridDim.x);
+}
+
+template <typename T>
+void launch_svd_load(const cplx_t<T>* a, int R, int N, cplx_t<T>* W, int ld, cudaStream_t s) {
+    k_svd_load<T><<<dim3((N + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(a, R, N, W, ld);
+    TQ_CHECK(cudaGetLastError());
+}
+
+template <typename T>
+void launch_svd_u(const cplx_t<T>* W, int ld, const int* perm, const double* sig, int R, int k, cplx_t<T>* u,
+                  cudaStream_t s) {
+    k_svd_u<T><<<dim3((k + 31) / 32, (R + 31) / 32), dim3(32, 8), 0, s>>>(W, ld, perm, sig, R, k, u);
+    TQ_CHECK(cudaGetLastError());
+}
+
+template <typename T>
+void launch_svd_vh(const cplx_t<T>* u, const cplx_t<T>* a, const double* sig, int R, int k, int N, cplx_t<T>* vh,
+                   cudaStream_t s) {
+    k_svd_vh<T><<<((k + 31) / 32) * ((N + 31) / 32), 256, 0, s>>>(u, a, sig, R, k, N, vh);
+    TQ_CHECK(cudaGetLastError());
+}
+
 template <typename T>
 __device__ void chain_body(const MpsView<T>& mps, int right, const ChainStep* steps, int nsteps, cplx_t<T>* envs,
                            cplx_t<T>* X, GridBar* bar, RunStats* stats, int cta, int ncta) {
@@ -3631,6 +3698,11 @@ void launch_entropy_batch(const InstTask<T>* insts, int ninst, cudaStream_t s) {
     template void launch_single_site<T>(const MpsView<T>&, const ScheduleView&, int, cudaStream_t);         \
     template void launch_theta<T>(const MpsView<T>&, const ScheduleView&, GateOp, const double*, SvdWork<T>, \
                                   int, int, cudaStream_t);                                                  \
+    template void launch_svd_load<T>(const cplx_t<T>*, int, int, cplx_t<T>*, int, cudaStream_t);            \
+    template void launch_svd_u<T>(const cplx_t<T>*, int, const int*, const double*, int, int, cplx_t<T>*,   \
+                                  cudaStream_t);                                                            \
+    template void launch_svd_vh<T>(const cplx_t<T>*, const cplx_t<T>*, const double*, int, int, int,        \
+                                   cplx_t<T>*, cudaStream_t);                                               \
     template bool svd_resident<T>(int, int);                                                                \
     template int launch_svd<T>(const MpsView<T>&, int, int, double, int, SvdWork<T>, int, int, int,         \
                                cudaStream_t, int, int, int, int);                                           \
