@@ -11,18 +11,21 @@
 // pattern (quantum.rs:94-103) and the sign<Z> pattern, with energies and probabilities.
 //
 // Layout: psi is 2^n complex128 in HBM (16 GiB at n = 30), diag_full and diag_zz 2^n doubles.
-// Single-qubit gates are applied in tiles: a CTA loads the 2^(5+K) amplitudes that share all
-// bits outside {0..4} and K target qubits (the low five bits keep the loads coalesced), applies
-// the gates of every target in shared memory, and writes the tile back -- one HBM round trip per
-// pass instead of one per qubit.  Passes cover qubits 0..11, then the rest in even groups of at
-// most seven (n = 24: three passes per half step).  The diagonal phases ride on the first pass's
-// load and the last pass's store, and the last pass of a step also sums the qubit-0 reduced
-// density matrix over its tile, so a mode-0 step is exactly one sweep of passes (three round
+// Single-qubit gates are applied in tiles of 2^12 amplitudes (n >= 12): a CTA loads the amplitudes
+// that share all bits outside the tile's, applies the gates of the tile's target qubits, and writes
+// the tile back -- one HBM round trip per pass instead of one per qubit.  A thread holds 16
+// amplitudes, four tile bits, in registers and applies those bits' gates there; shared memory only
+// changes which four bits are the registers'.  The first pass covers qubits 0..11, the rest go in
+// even groups of at most seven (n = 24: three passes per half step).  The diagonal phases ride on
+// the first pass's load and the last pass's store, and the last pass of a step also sums the qubit-0
+// reduced density matrix over its tile, so a mode-0 step is exactly one sweep of passes (three round
 // trips of psi at n = 24).  In mode 1 the closing single-qubit half step of one step and the
 // opening one of the next are merged into one gate per qubit, so that mode too costs one sweep
-// per step (plus one).
+// per step (plus one).  The gates of many sweeps are made by one launch, and the entropies of many
+// steps by one, so a step launches its passes and nothing else.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstdint>
 #include <cstring>
@@ -47,6 +50,9 @@ constexpr int SV_LOW = 5;         // low bits always in a tile
 constexpr int SV_TGT = 7;         // at most this many target qubits per tile above the low bits
 constexpr int SV_NT = 256;
 constexpr int SV_MAXN = 30;
+constexpr int SV_TILE = 12;       // tile bits from n = 12 on: 256 threads x 16 amplitudes
+constexpr int SV_SWEEPS = 256;    // sweeps whose gates one launch makes
+constexpr size_t SV_RHO_BYTES = 32u << 20;  // qubit-0 partial sums kept before an entropy launch
 
 struct SvPass {
     int nt;            // tile bits (low + targets)
@@ -102,11 +108,15 @@ __device__ void sv_gate(const double* h, const double* sa, const double* sb, con
     }
 }
 
-// Gate of every qubit for step k, or, with k2 >= 0, the product G(k2) G(k) (G(k) applied first).
+// Gates of every qubit for sweeps q0 + blockIdx.y.  Mode 0: sweep q is step q's.  Mode 1: sweep 0 opens
+// step 0, sweep q > 0 closes step q - 1 and opens step q (the product G(q) G(q - 1), G(q - 1) first;
+// none to open after the last).
 __global__ void k_sv_gates(const double* h, const double* sa, const double* sb, const double* bias, const double* sc,
-                           int n, int k, int k2, double dt, int mode, double2* gates) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+                           int n, int q0, int steps, double dt, int mode, double2* table) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, q = q0 + blockIdx.y;
     if (i >= n) return;
+    const int k = mode == 0 || q == 0 ? q : q - 1, k2 = mode == 1 && q > 0 && q < steps ? q : -1;
+    double2* gates = table + (size_t)4 * n * blockIdx.y;
     double2 g[4];
     sv_gate(h, sa, sb, bias, sc, i, k, dt, mode, g);
     if (k2 >= 0) {
@@ -118,7 +128,7 @@ __global__ void k_sv_gates(const double* h, const double* sa, const double* sb, 
                 gates[4 * i + 2 * r + c] = make_double2(x.x + y.x, x.y + y.y);
             }
     } else {
-        for (int q = 0; q < 4; ++q) gates[4 * i + q] = g[q];
+        for (int q4 = 0; q4 < 4; ++q4) gates[4 * i + q4] = g[q4];
     }
 }
 
@@ -134,14 +144,151 @@ __device__ __forceinline__ double2 sv_phase(double2 v, const SvPhase& ph, unsign
     return zmul(v, make_double2(cs, sn));
 }
 
-// One tiled pass of single-qubit gates, with an optional diagonal phase applied on load (pre)
-// and before the store (post), and optional partial sums of the qubit-0 reduced density matrix
-// (r00, r11, Re r01, Im r01 per CTA into rho) of the gated tile: after the post phase, or
-// before it when rho_first is set.
+// A pass over tiles of 12 bits: x bits 0..nlow-1 are tile bits 0..nlow-1, tile bit b above them is x
+// bit pos[b].  qubit[b]: the qubit whose gate acts on tile bit b, or -1.
+struct SvTile {
+    int nlow;
+    int pos[SV_TILE];
+    int qubit[SV_TILE];
+    int nrest;
+    int rpos[SV_MAXN];  // x bits outside the tile, ascending
+};
+
+// partial sums of the qubit-0 density matrix over the CTA, into rho
+__device__ __forceinline__ void sv_rho_out(double a, double b, double cr, double ci, double* rho) {
+    __shared__ double red[4][SV_NT / 32];
+    a = warp_sum(a); b = warp_sum(b); cr = warp_sum(cr); ci = warp_sum(ci);
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) { red[0][w] = a; red[1][w] = b; red[2][w] = cr; red[3][w] = ci; }
+    __syncthreads();
+    if (threadIdx.x < 4) {
+        double sum = 0;
+        for (int q = 0; q < SV_NT / 32; ++q) sum += red[threadIdx.x][q];
+        rho[4 * (size_t)blockIdx.x + threadIdx.x] = sum;
+    }
+}
+
+// the gates of tile bits tb .. tb + 3, which are the bits of j in v[j]
+__device__ __forceinline__ void sv_reg_gates(double2 (&v)[16], const SvTile& ps, const double2* gates, int tb) {
+#pragma unroll
+    for (int b = 0; b < 4; ++b) {
+        const int q = ps.qubit[tb + b];
+        if (q < 0) continue;
+        const double2* g = gates + 4 * q;
+        const double2 u00 = g[0], u01 = g[1], u10 = g[2], u11 = g[3];
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            if (j & (1 << b)) continue;
+            const double2 x = v[j], y = v[j | (1 << b)];
+            double2 p = zmul(u00, x), r = zmul(u10, x);
+            cfma(p, u01, y);
+            cfma(r, u11, y);
+            v[j] = p;
+            v[j | (1 << b)] = r;
+        }
+    }
+}
+
+// One pass, NS register stages: tile bits 8..11, then 4..7, then 0..3 (NS = 3: the first pass, whose
+// tile is then turned back so that the store is coalesced).  Phases and density-matrix sums as in
+// k_sv_pass.  Shared memory is padded by one amplitude in 16, which leaves every stage's access free
+// of bank conflicts.  Bound: FP64 issue (8 multiply-adds per amplitude and gate, a sincos per phase)
+// and a pass that loads, computes and stores with two CTAs an SM to overlap.  n = 22 (67 MB, in L2):
+// 52 us a pass against 88 us with every gate a shared-memory round and a barrier; 40 mode-1 steps 12.3
+// -> 7.1 ms.
+template <int NS>
+__global__ void __launch_bounds__(SV_NT, 2) k_sv_tile(double2* psi, SvTile ps, const double2* gates, SvPhase pre,
+                                                      SvPhase post, double* rho, int rho_first) {
+    extern __shared__ double2 tile[];
+    const int t = threadIdx.x;
+    unsigned long long base = 0, r = blockIdx.x;
+    for (int b = 0; b < ps.nrest; ++b, r >>= 1)
+        if (r & 1ull) base |= 1ull << ps.rpos[b];
+    // x index of register j in the layout whose register bits are tb .. tb + 3
+    auto thread_x = [&](int tb) {
+        const int i = (t & ((1 << tb) - 1)) | ((t >> tb) << (tb + 4));
+        unsigned long long x = base;
+#pragma unroll
+        for (int b = 0; b < SV_TILE; ++b)
+            if ((i >> b) & 1) x |= 1ull << ps.pos[b];
+        return x;
+    };
+    auto reg_x = [&](int tb, int j) {
+        unsigned long long x = 0;
+#pragma unroll
+        for (int b = 0; b < 4; ++b)
+            if ((j >> b) & 1) x |= 1ull << ps.pos[tb + b];
+        return x;
+    };
+    double2 v[16];
+    const unsigned long long x8 = thread_x(8);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = psi[x8 | reg_x(8, j)];
+    if (pre.d) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = sv_phase(v[j], pre, x8 | reg_x(8, j));
+    }
+    sv_reg_gates(v, ps, gates, 8);
+    // hand the tile over from register bits `from` to register bits `to`
+    auto turn = [&](int from, int to) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int i = (t & ((1 << from) - 1)) | (j << from) | ((t >> from) << (from + 4));
+            tile[i + (i >> 4)] = v[j];
+        }
+        __syncthreads();
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const int i = (t & ((1 << to) - 1)) | (j << to) | ((t >> to) << (to + 4));
+            v[j] = tile[i + (i >> 4)];
+        }
+    };
+    if (NS >= 2) {
+        turn(8, 4);
+        sv_reg_gates(v, ps, gates, 4);
+    }
+    if (NS >= 3) {
+        __syncthreads();
+        turn(4, 0);
+        sv_reg_gates(v, ps, gates, 0);
+        __syncthreads();
+        turn(0, 8);
+    }
+    constexpr int TB = NS == 2 ? 4 : 8;
+    const unsigned long long xo = NS == 2 ? thread_x(TB) : x8;
+    auto sums = [&]() {  // x bit 0 is a lane's lowest bit: its partner in qubit 0 is the next lane
+        double a = 0, b = 0, cr = 0, ci = 0;
+#pragma unroll
+        for (int j = 0; j < 16; ++j) {
+            const double wx = __shfl_xor_sync(0xffffffffu, v[j].x, 1), wy = __shfl_xor_sync(0xffffffffu, v[j].y, 1);
+            const double nv = v[j].x * v[j].x + v[j].y * v[j].y;
+            if (t & 1) {
+                b += nv;
+            } else {
+                a += nv;
+                cr += v[j].x * wx + v[j].y * wy;  // u conj(v)
+                ci += v[j].y * wx - v[j].x * wy;
+            }
+        }
+        sv_rho_out(a, b, cr, ci, rho);
+    };
+    if (rho && (rho_first || !post.d)) sums();
+    if (post.d) {
+#pragma unroll
+        for (int j = 0; j < 16; ++j) v[j] = sv_phase(v[j], post, xo | reg_x(TB, j));
+        if (rho && !rho_first) sums();
+    }
+#pragma unroll
+    for (int j = 0; j < 16; ++j) psi[xo | reg_x(TB, j)] = v[j];
+}
+
+// One pass of single-qubit gates over a tile in shared memory (n < 12: the whole state), with an
+// optional diagonal phase applied on load (pre) and before the store (post), and optional partial
+// sums of the qubit-0 reduced density matrix (r00, r11, Re r01, Im r01 per CTA into rho) of the gated
+// tile: after the post phase, or before it when rho_first is set.
 __global__ void __launch_bounds__(SV_NT) k_sv_pass(double2* psi, SvPass ps, const double2* gates, SvPhase pre,
                                                    SvPhase post, double* rho, int rho_first) {
     extern __shared__ double2 tile[];
-    __shared__ double red[4][SV_NT / 32];
     const int T = 1 << ps.nt;
     // base index of this CTA: blockIdx spread over the rest bits
     unsigned long long base = 0, r = blockIdx.x;
@@ -191,15 +338,7 @@ __global__ void __launch_bounds__(SV_NT) k_sv_pass(double2* psi, SvPass ps, cons
             cr += u.x * v.x + u.y * v.y;  // u conj(v)
             ci += u.y * v.x - u.x * v.y;
         }
-        a = warp_sum(a); bb = warp_sum(bb); cr = warp_sum(cr); ci = warp_sum(ci);
-        const int w = threadIdx.x >> 5;
-        if ((threadIdx.x & 31) == 0) { red[0][w] = a; red[1][w] = bb; red[2][w] = cr; red[3][w] = ci; }
-        __syncthreads();
-        if (threadIdx.x < 4) {
-            double sum = 0;
-            for (int q = 0; q < SV_NT / 32; ++q) sum += red[threadIdx.x][q];
-            rho[4 * (size_t)blockIdx.x + threadIdx.x] = sum;
-        }
+        sv_rho_out(a, bb, cr, ci, rho);
     }
     const bool post_on_store = post.d && !post_in_tile;
     for (int t = threadIdx.x; t < T; t += SV_NT) {
@@ -210,7 +349,9 @@ __global__ void __launch_bounds__(SV_NT) k_sv_pass(double2* psi, SvPass ps, cons
     }
 }
 
-__global__ void k_sv_entropy(const double* part, int nblk, double* out, int k) {
+// entropies of steps k + blockIdx.x from their partial sums
+__global__ void k_sv_entropy(const double* parts, int nblk, double* out, int k) {
+    const double* part = parts + 4 * (size_t)nblk * blockIdx.x;
     __shared__ double red[4][SV_NT / 32];
     double r[4] = {0, 0, 0, 0};
     for (int b = threadIdx.x; b < nblk; b += blockDim.x)
@@ -231,7 +372,7 @@ __global__ void k_sv_entropy(const double* part, int nblk, double* out, int k) {
         if (l1 > 1e-12) S -= l1 * log2(l1);
         if (l2 > 1e-12) S -= l2 * log2(l2);
     }
-    out[k] = S;
+    out[k + blockIdx.x] = S;
 }
 
 // per-block: total probability, sum p E(x), best p and its (smallest) index, sum p z_i
@@ -284,7 +425,45 @@ __global__ void k_sv_final(const double2* psi, const double* dfull, unsigned lon
     }
 }
 
-// Passes of one half step: the first gates the low bits and the next SV_TGT qubits; the rest
+// Passes from n = 12 on: qubits 0..11, then the rest in even groups of at most SV_TGT.  A group of g
+// targets is tile bits 12-g..11 (8..11 when g < 4, the rest of those being any other qubits).
+static std::vector<SvTile> plan_tiles(int n) {
+    std::vector<SvTile> out;
+    const int rem = n - SV_TILE;
+    const int np = 1 + (rem > 0 ? (rem + SV_TGT - 1) / SV_TGT : 0);
+    int q = SV_TILE;
+    for (int pi = 0; pi < np; ++pi) {
+        SvTile p{};
+        std::vector<int> tgt;
+        int g = SV_TILE;
+        if (pi > 0) {
+            g = rem / (np - 1) + (pi - 1 < rem % (np - 1) ? 1 : 0);
+            for (int c = 0; c < g; ++c) tgt.push_back(q++);
+        }
+        p.nlow = pi == 0 ? SV_TILE : SV_TILE - (g < 4 ? 4 : g);
+        for (int b = 0; b < SV_TILE; ++b) {
+            p.pos[b] = b;
+            p.qubit[b] = pi == 0 ? b : -1;
+        }
+        if (pi > 0) {
+            int b = p.nlow, fill = p.nlow;
+            for (; SV_TILE - b > g; ++b) p.pos[b] = fill++;  // fillers: the next low bits, not gated
+            for (int t : tgt) {
+                p.pos[b] = t;
+                p.qubit[b++] = t;
+            }
+        }
+        for (int x = 0; x < n; ++x) {
+            bool in = false;
+            for (int b = 0; b < SV_TILE; ++b) in = in || p.pos[b] == x;
+            if (!in) p.rpos[p.nrest++] = x;
+        }
+        out.push_back(p);
+    }
+    return out;
+}
+
+// Passes below n = 12 (one, in effect): the first gates the low bits and the next SV_TGT qubits; the rest
 // are spread evenly over as few passes as hold at most SV_TGT targets each (no small last pass).
 static std::vector<SvPass> plan_passes(int n) {
     std::vector<SvPass> out;
@@ -370,15 +549,21 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         const int grid = nsm * 8;
         char* arena = nullptr;
         auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
+        const bool tiled = n >= SV_TILE;
+        const std::vector<SvPass> passes = tiled ? std::vector<SvPass>() : plan_passes(n);
+        const std::vector<SvTile> tiles = tiled ? plan_tiles(n) : std::vector<SvTile>();
+        // qubit-0 partials: one set per last-pass CTA, kept for `held` steps
+        const size_t rho_blocks = 1ull << (tiled ? tiles.back().nrest : passes.back().nrest);
+        const int held = (int)std::max<size_t>(1, std::min<size_t>(steps, SV_RHO_BYTES / (32 * rho_blocks)));
+        const int sweeps = mode == 0 ? steps : steps + 1;
+        const int made = std::min(sweeps, SV_SWEEPS);  // sweeps whose gates are made at a time
         const size_t o_psi = 0, o_df = o_psi + al(dim * 16), o_dz = o_df + al(dim * 8);
         const size_t o_h = o_dz + al(dim * 8), o_w = o_h + al(8 * n), o_i = o_w + al(8 * (m + 1));
         const size_t o_j = o_i + al(4 * (m + 1)), o_sa = o_j + al(4 * (m + 1)), o_sb = o_sa + al(8 * steps);
         const size_t o_bias = o_sb + al(8 * steps), o_sc = o_bias + al(8 * n), o_g = o_sc + al(8 * steps);
-        const size_t o_part = o_g + al(64 * n), o_ent = o_part + al(8 * (size_t)grid * (3 + SV_MAXN));
-        const std::vector<SvPass> passes = plan_passes(n);
-        const size_t rho_blocks = 1ull << passes.back().nrest;  // qubit-0 partials: one set per last-pass CTA
+        const size_t o_part = o_g + al((size_t)64 * n * made), o_ent = o_part + al(8 * (size_t)grid * (3 + SV_MAXN));
         const size_t o_bx = o_ent + al(8 * steps), o_rho = o_bx + al(8 * (size_t)grid);
-        const size_t total = o_rho + al(32 * rho_blocks);
+        const size_t total = o_rho + al(32 * rho_blocks * held);
         SV_CK(device_alloc((void**)&arena, total));
         auto at = [&](size_t o) { return arena + o; };
         double2* psi = (double2*)at(o_psi);
@@ -406,39 +591,53 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         cudaEvent_t e0, e1;
         if (err == cudaSuccess) err = cudaEventCreate(&e0);
         if (err == cudaSuccess) err = cudaEventCreate(&e1);
-        int maxnt = 0;
-        for (const SvPass& p : passes) maxnt = p.nt > maxnt ? p.nt : maxnt;
-        const size_t tile_bytes = sizeof(double2) << maxnt;
-        if (err == cudaSuccess && tile_bytes > 48 * 1024)
-            err = cudaFuncSetAttribute(k_sv_pass, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
+        const size_t tile_bytes = tiled ? (sizeof(double2) << SV_TILE) / 16 * 17 : sizeof(double2) << passes[0].nt;
+        if (err == cudaSuccess && tiled) {
+            err = cudaFuncSetAttribute(k_sv_tile<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
+            if (err == cudaSuccess)
+                err = cudaFuncSetAttribute(k_sv_tile<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
+        }
         if (err == cudaSuccess) err = cudaMemsetAsync(dent, 0, 8 * (size_t)steps, st);  // n = 1: no entanglement
         if (err == cudaSuccess) {
             cudaEventRecord(e0, st);
             k_sv_diag<<<grid, SV_NT, 0, st>>>(dh, di, dj, dw, n, m, dim, df, dz, psi);
             const SvPhase none{nullptr, 0.0};
             const double* hsb = P->schedule_b;
-            auto gates = [&](int k, int k2) {
-                k_sv_gates<<<(n + 63) / 64, 64, 0, st>>>(dh, dsa, dsb, P->bias ? dbias : nullptr, dsc, n, k, k2, dt,
-                                                        mode, dg);
-            };
-            // One sweep of the gate passes; `pre` rides on the first pass's load, `post` and the
-            // qubit-0 partial sums on the last pass.
-            auto sweep = [&](SvPhase pre, SvPhase post, double* rho, int rho_first) {
+            // Sweep q of the gate passes; `pre` rides on the first pass's load, `post` and the qubit-0
+            // partial sums on the last pass.
+            auto sweep = [&](int q, SvPhase pre, SvPhase post, double* rho, int rho_first) {
+                if (q % made == 0)
+                    k_sv_gates<<<dim3((n + 63) / 64, std::min(made, sweeps - q)), 64, 0, st>>>(
+                        dh, dsa, dsb, P->bias ? dbias : nullptr, dsc, n, q, steps, dt, mode, dg);
+                const double2* g = dg + (size_t)4 * n * (q % made);
+                for (size_t i = 0; i < tiles.size(); ++i) {
+                    const SvTile& p = tiles[i];
+                    const bool last = i + 1 == tiles.size();
+                    const unsigned blocks = 1u << p.nrest;
+                    const SvPhase a0 = i == 0 ? pre : none, a1 = last ? post : none;
+                    double* ro = last ? rho : nullptr;
+                    if (i == 0) k_sv_tile<3><<<blocks, SV_NT, tile_bytes, st>>>(psi, p, g, a0, a1, ro, rho_first);
+                    else if (p.nlow < 8) k_sv_tile<2><<<blocks, SV_NT, tile_bytes, st>>>(psi, p, g, a0, a1, ro, rho_first);
+                    else k_sv_tile<1><<<blocks, SV_NT, 0, st>>>(psi, p, g, a0, a1, ro, rho_first);
+                }
                 for (size_t i = 0; i < passes.size(); ++i) {
                     const SvPass& p = passes[i];
                     const bool last = i + 1 == passes.size();
-                    const unsigned long long blocks = 1ull << p.nrest;
-                    k_sv_pass<<<(unsigned)blocks, SV_NT, sizeof(double2) << p.nt, st>>>(
-                        psi, p, dg, i == 0 ? pre : none, last ? post : none, last ? rho : nullptr, rho_first);
+                    k_sv_pass<<<1u << p.nrest, SV_NT, sizeof(double2) << p.nt, st>>>(
+                        psi, p, g, i == 0 ? pre : none, last ? post : none, last ? rho : nullptr, rho_first);
                 }
             };
-            double* rho = n >= 2 ? drho : nullptr;
+            // partial sums of step k, and its entropy with those of the steps held before it
+            auto rho_of = [&](int k) { return n >= 2 ? drho + 4 * rho_blocks * (k % held) : nullptr; };
+            auto entropies = [&](int k) {
+                if (n >= 2 && (k % held == held - 1 || k + 1 == steps))
+                    k_sv_entropy<<<k % held + 1, SV_NT, 0, st>>>(drho, (int)rho_blocks, dent, k - k % held);
+            };
             if (mode == 0) {  // P X P per step: one sweep, both phases fused into it
                 for (int k = 0; k < steps; ++k) {
                     const SvPhase ph{df, 0.5 * hsb[k] * dt};
-                    gates(k, -1);
-                    sweep(ph, ph, rho, 0);
-                    if (rho) k_sv_entropy<<<1, SV_NT, 0, st>>>(rho, (int)rho_blocks, dent, k);
+                    sweep(k, ph, ph, rho_of(k), 0);
+                    entropies(k);
                 }
             } else {
                 // G(k) Z(k) G(k) per step.  The closing half step of step k and the opening one of
@@ -446,13 +645,11 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
                 // the products G(k+1) G(k).  The qubit-0 entropy of step k is read from that
                 // sweep before the next ZZ phase: G(k+1) is a product of one-qubit unitaries,
                 // which leaves the Schmidt spectrum across the qubit-0 cut unchanged.
-                gates(0, -1);
-                sweep(none, SvPhase{dz, 1.0 * hsb[0] * dt}, nullptr, 0);
+                sweep(0, none, SvPhase{dz, 1.0 * hsb[0] * dt}, nullptr, 0);
                 for (int k = 0; k < steps; ++k) {
                     const bool more = k + 1 < steps;
-                    gates(k, more ? k + 1 : -1);
-                    sweep(none, more ? SvPhase{dz, 1.0 * hsb[k + 1] * dt} : none, rho, 1);
-                    if (rho) k_sv_entropy<<<1, SV_NT, 0, st>>>(rho, (int)rho_blocks, dent, k);
+                    sweep(k + 1, none, more ? SvPhase{dz, 1.0 * hsb[k + 1] * dt} : none, rho_of(k), 1);
+                    entropies(k);
                 }
             }
             k_sv_final<<<grid, SV_NT, 0, st>>>(psi, df, dim, n, part, dbx);
