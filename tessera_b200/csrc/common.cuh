@@ -8,7 +8,8 @@ namespace tq {
 // Every device allocation of the library goes through here (engine.cu): the library's memory
 // pool, except that tessera_qa_debug_fail_allocations(after, count) makes chosen calls fail with
 // cudaErrorMemoryAllocation, so the out-of-memory paths can be tested without exhausting a GPU.
-cudaError_t device_alloc(void** p, size_t bytes);
+// pooled: the memory lives for one call of the library.
+cudaError_t device_alloc(void** p, size_t bytes, bool pooled = false);
 // Back to the pool; the work that used it has been waited for.
 void device_free(void* p);
 void device_trim();  // what the pool holds unused on the current device, back to the driver

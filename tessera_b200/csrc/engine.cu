@@ -53,10 +53,11 @@ static int g_fail_after = 0, g_fail_count = 0;
 // The library's own memory pool on each device.  cudaMalloc and cudaFree map and unmap pages and
 // wait for the whole device: on one box 0.1 ms a pair, on another 3 ms, and more for 100 MB, beside
 // kernels of a few microseconds; a call that makes an engine, runs it and drops it paid that several
-// times.  The pool holds at most kKeep bytes per device; an allocation that would take it further is
-// a plain cudaMalloc (148 arenas of 55 MB: 0.13 s through the pool, 0.09 s that way).  What the pool
-// holds unused goes back to the driver when an allocation fails or device_trim() is called, and the
-// pools end with the process.  Allocation and release run on a stream of the pool's own that no
+// times.  Only such calls use the pool (device_alloc's `pooled`): what a session or a network holds is
+// plain memory, as it is made once.  The pool holds at most kKeep bytes per device, grows by kGrow at a
+// time (a growth of a few MB per allocation made 100 small engines take 1 ms each), and an allocation
+// that would take it beyond kKeep is a plain cudaMalloc.  What the pool holds unused goes back to the
+// driver when an allocation fails or device_trim() is called, and the pools end with the process.  Allocation and release run on a stream of the pool's own that no
 // kernel uses, and are waited for, so the memory is good for any stream and thread when alloc()
 // returns; callers have waited for their work before they free, as cudaFree's callers had not to.
 class DevicePools {
@@ -65,13 +66,14 @@ public:
         static DevicePools* p = new DevicePools;  // never destroyed: engines may outlive static objects
         return *p;
     }
-    cudaError_t alloc(void** out, size_t bytes) {
+    cudaError_t alloc(void** out, size_t bytes, bool want) {
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
         std::lock_guard<std::mutex> lk(mu_);
         Pool* pl = pool(dev);
-        const bool pooled = pl && pl->used + bytes <= kKeep;
+        const bool pooled = want && pl && pl->used + bytes <= kKeep;
+        if (pooled) grow(*pl, bytes);
         for (int turn = 0; turn < 2; ++turn) {
             if (pooled) {
                 e = cudaMallocFromPoolAsync(out, bytes, pl->pool, pl->st);
@@ -113,6 +115,7 @@ public:
 private:
     static constexpr int kMax = 64;
     static constexpr uint64_t kKeep = 256ull << 20;
+    static constexpr uint64_t kGrow = 64ull << 20;
     struct Pool {
         int state = 0;  // 0 not tried, 1 ready, 2 not to be had on this device
         cudaMemPool_t pool = nullptr;
@@ -123,6 +126,16 @@ private:
         int dev;
         size_t bytes;
     };
+    // takes and returns a block of kGrow when the next allocation would make the pool grow
+    void grow(Pool& pl, size_t bytes) {
+        uint64_t held = 0;
+        if (bytes >= kGrow || cudaMemPoolGetAttribute(pl.pool, cudaMemPoolAttrReservedMemCurrent, &held) != cudaSuccess ||
+            pl.used + bytes <= held || held + kGrow > kKeep)
+            return;
+        void* p = nullptr;
+        if (cudaMallocFromPoolAsync(&p, kGrow, pl.pool, pl.st) == cudaSuccess) cudaFreeAsync(p, pl.st);
+        else cudaGetLastError();
+    }
     Pool* pool(int dev) {  // dev is current; nullptr: plain cudaMalloc
         if (dev < 0 || dev >= kMax) return nullptr;
         Pool& pl = pools_[dev];
@@ -150,7 +163,7 @@ private:
     std::unordered_map<void*, Block> owner_;
 };
 
-cudaError_t device_alloc(void** p, size_t bytes) {
+cudaError_t device_alloc(void** p, size_t bytes, bool pooled) {
     {
         std::lock_guard<std::mutex> lk(g_fail_mu);
         if (g_fail_count > 0) {
@@ -163,7 +176,7 @@ cudaError_t device_alloc(void** p, size_t bytes) {
             }
         }
     }
-    return DevicePools::get().alloc(p, bytes);
+    return DevicePools::get().alloc(p, bytes, pooled);
 }
 void device_free(void* p) { DevicePools::get().free(p); }
 void device_trim() { DevicePools::get().trim(); }
@@ -264,6 +277,7 @@ struct Config {
     int min_ld = 0;  // workspace rows/cols at least this (standalone SVD)
     int timing = 0;  // time each SVD launch with CUDA events
     int theta_tc = 0;  // complex64: bond contraction on tcgen05 tensor cores (split-TF32)
+    bool pooled = false;  // device memory from the pool: the engine lives for one call
     int precond = 0;   // batched column-pair Jacobi: 0 default (on), 1 on, 2 off (pivoted LQ first)
 };
 
@@ -565,7 +579,7 @@ public:
     void ensure_obs() {
         if (obs_) return;
         const size_t bytes = sizeof(V) * (size_t)cap_ * cap_ * obs_units_;
-        TQ_CK(device_alloc((void**)&obs_, bytes));
+        TQ_CK(device_alloc((void**)&obs_, bytes, C_.pooled));
         TQ_CK(cudaMemsetAsync(obs_, 0, sizeof(V), stream_));
         V one = mk<V>(1, 0);
         TQ_CK(cudaMemcpyAsync(obs_, &one, sizeof(V), cudaMemcpyHostToDevice, stream_));
@@ -608,7 +622,7 @@ public:
         ensure_obs();
         launch_chain<T>(M, 1, obsR_, n_, obs_, xs_, bar_, stats_, cap_, stream_);
         int8_t* d = nullptr;
-        TQ_CK(device_alloc((void**)&d, count * (size_t)n_));
+        TQ_CK(device_alloc((void**)&d, count * (size_t)n_, true));
         cudaError_t err = cudaSuccess;
         try {
             launch_sample<T>(M, obs_, (int)count, seed, d, stream_);
@@ -718,7 +732,7 @@ public:
             }
         } buf;
         buf.st = stream_;
-        TQ_CK(device_alloc((void**)&buf.p, na + nu + align256(sizeof(V) * (size_t)k * N)));
+        TQ_CK(device_alloc((void**)&buf.p, na + nu + align256(sizeof(V) * (size_t)k * N), true));
         V* da = reinterpret_cast<V*>(buf.p);
         V* du = reinterpret_cast<V*>(buf.p + na);
         V* dv = reinterpret_cast<V*>(buf.p + na + nu);
@@ -792,7 +806,7 @@ public:
         if (res_base_) return;
         const size_t a1 = align256(sizeof(InstTask<T>));
         const size_t a2 = a1 + align256(sizeof(GateOp) * std::max<size_t>(ops_.size(), 1));
-        TQ_CK(device_alloc((void**)&res_base_, a2 + 256));
+        TQ_CK(device_alloc((void**)&res_base_, a2 + 256, C_.pooled));
         res_inst_ = reinterpret_cast<InstTask<T>*>(res_base_);
         res_ops_ = reinterpret_cast<GateOp*>(res_base_ + a1);
         res_off_ = reinterpret_cast<int*>(res_base_ + a2);
@@ -946,7 +960,7 @@ private:
         lq_ok_ = ld_ > (sizeof(T) == 8 ? 64 : 256) && ld_ <= 1024;
         add((void**)&lqc_, lq_ok_ ? lq_coop_scratch_bytes(ld_, (int)es, (ld_ + 7) / 8) : 8);
         TQ_CK(cudaStreamCreateWithFlags(&stream_, cudaStreamNonBlocking));
-        TQ_CK(device_alloc((void**)&base_, off));
+        TQ_CK(device_alloc((void**)&base_, off, C_.pooled));
         for (auto& it : plan) *it.second = base_ + it.first;
         TQ_CK(cudaMemsetAsync(bar_, 0, sizeof(GridBar), stream_));
         TQ_CK(cudaMemsetAsync(stats_, 0, sizeof(RunStats), stream_));
@@ -1199,7 +1213,7 @@ private:
         const size_t a3 = a2 + align256(sizeof(GateOp) * std::max<size_t>(ops_all.size(), 1));
         const size_t a4 = a3 + align256(sizeof(int) * (B + 1));
         const size_t bytes = a4 + align256(sizeof(int) * B);
-        TQ_CK(device_alloc((void**)&base_, bytes));
+        TQ_CK(device_alloc((void**)&base_, bytes, C[0].pooled));
         step_ = reinterpret_cast<int*>(base_);
         work_ = reinterpret_cast<int*>(base_ + 64);
         insts_ = reinterpret_cast<InstTask<T>*>(base_ + a0);
@@ -1398,7 +1412,7 @@ public:
             }
         } buf;
         buf.st = st_;
-        TQ_CK(device_alloc((void**)&buf.p, o_s + align256(nspins)));
+        TQ_CK(device_alloc((void**)&buf.p, o_s + align256(nspins), true));
         ObsTask<T>* dt = reinterpret_cast<ObsTask<T>*>(buf.p);
         double *dv = reinterpret_cast<double*>(buf.p + o_v), *da = reinterpret_cast<double*>(buf.p + o_a);
         int8_t* ds = reinterpret_cast<int8_t*>(buf.p + o_s);
@@ -1575,6 +1589,7 @@ int tessera_qa_anneal_ex(const tessera_qa_problem* problem, const tessera_qa_con
         if (!result) throw ArgError("result is NULL");
         ProblemHost P = validate_problem(problem);
         Config C = validate_config(config);
+        C.pooled = true;
         const int k0 = config ? (int)config->step_begin : 0;
         const int k1 = (config && config->step_end) ? (int)config->step_end : P.steps;
         if (k0 > k1 || k1 > P.steps) throw ArgError("step range outside the schedule");
@@ -1606,6 +1621,7 @@ int tessera_qa_anneal_batch(const tessera_qa_problem* problems, const tessera_qa
         for (size_t b = 0; b < count; ++b) {
             P.push_back(validate_problem(&problems[b]));
             C.push_back(validate_config(&configs[b]));
+            C.back().pooled = true;
             if (C.back().precision != C[0].precision) throw ArgError("batched instances must share the precision");
             if (configs[b].initial_mps) throw ArgError("batched runs start from |+>^n");
         }
@@ -1670,6 +1686,7 @@ int tessera_qa_svd(const double* a, size_t rows, size_t cols, double* s, double*
         Config C;
         C.chi = 1;
         C.min_ld = std::max(R, N);
+        C.pooled = true;
         int dev = 0;
         if (cudaGetDeviceCount(&dev) != cudaSuccess || dev == 0) throw CudaError("no CUDA device available");
         Engine<double> eng(P, C);

@@ -297,7 +297,7 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
                      b_s = al(h.size()), b_part = al(sizeof(SaBest) * count * ctas), b_tick = al(sizeof(int) * count);
         const size_t total = b_tasks + b_off + b_nbr + b_w + b_h + 2 * b_ei + b_ew + b_e + b_s + b_part + b_tick;
         SA_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-        SA_CK(device_alloc((void**)&arena, total));
+        SA_CK(device_alloc((void**)&arena, total, true));
         char* q = arena;
         auto take = [&](size_t bytes) { char* r = q; q += bytes; return r; };
         SaTask* d_tasks = (SaTask*)take(b_tasks);

@@ -564,7 +564,7 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         const size_t o_part = o_g + al((size_t)64 * n * made), o_ent = o_part + al(8 * (size_t)grid * (3 + SV_MAXN));
         const size_t o_bx = o_ent + al(8 * steps), o_rho = o_bx + al(8 * (size_t)grid);
         const size_t total = o_rho + al(32 * rho_blocks * held);
-        SV_CK(device_alloc((void**)&arena, total));
+        SV_CK(device_alloc((void**)&arena, total, true));
         auto at = [&](size_t o) { return arena + o; };
         double2* psi = (double2*)at(o_psi);
         double *df = (double*)at(o_df), *dz = (double*)at(o_dz), *dh = (double*)at(o_h), *dw = (double*)at(o_w);
