@@ -465,8 +465,10 @@ __device__ __forceinline__ void tournament(int P, int r, int pr, int& I, int& J)
         I = Q;
         J = r;
     } else {
-        I = (r + pr) % Q;
-        J = (r - pr + Q) % Q;
+        I = r + pr;  // modulo Q (r and pr are below it): no division on the way to a round's loads
+        if (I >= Q) I -= Q;
+        J = r - pr;
+        if (J < 0) J += Q;
     }
 }
 
@@ -1255,12 +1257,16 @@ __device__ void jacobi_core_d(double2* col, const int rc, const int R, const int
                     gr = fma(x[k].x, y[k].x, fma(x[k].y, y[k].y, gr));
                     gi = fma(x[k].x, y[k].y, fma(-x[k].y, y[k].x, gi));
                 }
+                if constexpr (LPP == 32) {
+                    warp_sum4(a, b, gr, gi);
+                } else {
 #pragma unroll
-                for (int o = LPP / 2; o > 0; o >>= 1) {
-                    a += __shfl_xor_sync(0xffffffffu, a, o);
-                    b += __shfl_xor_sync(0xffffffffu, b, o);
-                    gr += __shfl_xor_sync(0xffffffffu, gr, o);
-                    gi += __shfl_xor_sync(0xffffffffu, gi, o);
+                    for (int o = LPP / 2; o > 0; o >>= 1) {
+                        a += __shfl_xor_sync(0xffffffffu, a, o);
+                        b += __shfl_xor_sync(0xffffffffu, b, o);
+                        gr += __shfl_xor_sync(0xffffffffu, gr, o);
+                        gi += __shfl_xor_sync(0xffffffffu, gi, o);
+                    }
                 }
                 double tr, ti;
                 if (ok && jacobi_tau(a, b, gr, gi, tol2, tiny, mixed, tr, ti)) {
@@ -1534,10 +1540,24 @@ __device__ void resident_update(const MpsView<T>& mps, const ScheduleView& sch, 
         const V* u = col + wk.perm[k] * rc;
         const V* t = wk.theta + (long long)j * ld;
         double re = 0.0, im = 0.0;
-        for (int row = 0; row < R; ++row) {
-            const V uu = u[row], tt = t[row];
-            re += (double)uu.x * tt.x + (double)uu.y * tt.y;
-            im += (double)uu.x * tt.y - (double)uu.y * tt.x;
+        if constexpr (sizeof(T) == 8) {  // four chains
+            double r1 = 0.0, i1 = 0.0;
+#pragma unroll 4
+            for (int row = 0; row < R; ++row) {
+                const V uu = u[row], tt = t[row];
+                re = fma(uu.x, tt.x, re);
+                r1 = fma(uu.y, tt.y, r1);
+                im = fma(uu.x, tt.y, im);
+                i1 = fma(-uu.y, tt.x, i1);
+            }
+            re += r1;
+            im += i1;
+        } else {
+            for (int row = 0; row < R; ++row) {
+                const V uu = u[row], tt = t[row];
+                re += (double)uu.x * tt.x + (double)uu.y * tt.y;
+                im += (double)uu.x * tt.y - (double)uu.y * tt.x;
+            }
         }
         const double inv = 1.0 / wk.sig[k];
         const int s2 = j >= dr ? 1 : 0, b = j - s2 * dr;
