@@ -347,7 +347,7 @@ def plain_rate(args, local, peak_gbs=None, peak_tflops=None):
                 "compute": {"achieved": tfl, "unit": "TFLOP/s", "peak": peak_tflops,
                             "frac": tfl / peak_tflops if peak_tflops else None},
                 "precond_avg_launch_ms": (r.precond_ms - r0.precond_ms) / n,
-                "precond": "k_lq_coop (cooperative pivoted LQ, 8 rows of theta per CTA)"
+                "precond": "k_lq_coop_block / k_lq_coop (cooperative pivoted LQ, 8 rows of theta per CTA)"
                            if args.precondition == "on" else "off"}
     return g / (r.device_ms / 1e3), r.device_ms / g, roof
 
@@ -628,16 +628,20 @@ def main():
                         "flops_per_launch": svd_flops / max(svd_n, 1)}
 
     # the pivoted-LQ preconditioner (k_lq_batch): its own launches, timed apart from the Jacobi;
-    # algorithmic bytes per theta: one read for the row norms, then per elimination step one read
-    # of the trailing block and one write of column k, and per panel of 8 steps one read and one
-    # write of the trailing block (the delayed updates)
+    # algorithmic bytes per theta: one read for the row norms, then in complex128 (panels of 16 rows,
+    # 512 columns at most) one read and one write of the trailing block per panel; in complex64 and
+    # beyond 512 columns per elimination step one read of the trailing block and one write of column
+    # k, and per panel of 8 steps one read and one write of the trailing block (the delayed updates)
     precond = None
     if B > 1 and args.precondition == "on" and lq_ms > 0:
         R = Nc = 2 * args.chi
         esz = 16 if args.precision == "c128" else 8
         km = min(R, Nc)
-        lq_bytes = esz * (R * Nc + sum((R - k) * (Nc - k) + (R - k) for k in range(km))
-                          + sum(2 * (R - k) * (Nc - k) for k in range(8, km + 1, 8)))
+        if args.precision == "c128" and Nc <= 512:
+            lq_bytes = esz * (R * Nc + sum(2 * (R - k) * (Nc - k) for k in range(0, km, 16)))
+        else:
+            lq_bytes = esz * (R * Nc + sum((R - k) * (Nc - k) + (R - k) for k in range(km))
+                              + sum(2 * (R - k) * (Nc - k) for k in range(8, km + 1, 8)))
         lq_per_launch = B * lq_bytes
         lq_avg = lq_ms / max(svd_n, 1)
         precond = {"kernel": "k_lq_batch (row-pivoted Householder LQ, one CTA per 512x512 theta)",

@@ -965,10 +965,11 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
     }
     if (!cta_sync(wk.bar, status, nblk)) return;
     if (cta != 0) return;
-    // pairs evaluated (16 flops per row: four FP64 dot products) and rotated (32 per row)
+    // flops per row of a pair evaluated and of one rotated: 16 and 32 (two norms, the inner product);
+    // with carried norms 8 and 20
     double rots = 0.0;
     for (int e = 0; e < sweep && e < pp.max_sweeps; ++e) rots += (double)(*(volatile int*)&wk.counters[e]);
-    const double flops = (double)sweep * 0.5 * N * (N - 1) * R * 16.0 + rots * R * 32.0;
+    const double flops = (double)sweep * 0.5 * N * (N - 1) * R * (D ? 8.0 : 16.0) + rots * R * (D ? 20.0 : 32.0);
     svd_finish<T>(mps, wk, pp, R, N, keep_floor, sweep, converged,
                   ((double)sweep * (P - 1) * 2.0 + 2.0) * (double)R * N * sizeof(V), smraw, red, flops);
 }
@@ -978,12 +979,13 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
 // memory (column c at col + c * rows_cap) for the entire SVD, so there is no staging and
 // no block structure: every round of the circle method over all N columns rotates N/2
 // disjoint pairs.  A pair is owned by LPP lanes (RPL complex rows per lane, R <= LPP RPL),
-// so a warp rotates 32/LPP pairs at once and the reduction is log2(LPP) shuffle levels;
-// alpha, beta, gamma are accumulated and reduced in FP64 and the rotation is
-// jacobi_rotation's.  A sweep is N-1 rounds; a sweep without a rotation ends the
-// iteration.  Up to 8 register rows per lane (fewer in use for small R) and LPP by size
-// class: 8 up to R = 64, 16 up to 128, 32 up to 256.  One instantiation serves a whole class,
-// so a theta is rotated by the same instructions whatever batch it runs in.
+// so a warp rotates 32/LPP pairs at once and the reduction is log2(LPP) shuffle levels.
+// A sweep is N-1 rounds; a sweep without a rotation ends the iteration.  LPP by size class:
+// 8 up to R = 64, 16 up to 128, 32 up to 256.  One instantiation serves a whole class, so a
+// theta is rotated by the same instructions whatever batch it runs in.
+// complex64 (jacobi_core): up to 8 register rows per lane; alpha, beta, gamma are FP32 lane sums
+// reduced in FP64 and the rotation is jacobi_rotation's.  complex128: lq_resident, then
+// jacobi_core_d over its rank.
 // ------------------------------------------------------------------------------------
 constexpr int RES_MAXT = 512;
 constexpr int RES_RPL = 8;  // register rows per lane; R <= LPP * RES_RPL
@@ -1027,25 +1029,13 @@ __device__ void jacobi_core(cplx_t<T>* col, const int rc, const int R, const int
                     x[k] = in ? cp[row] : czero<V>();
                     y[k] = in ? cq[row] : czero<V>();
                 }
-                double v0 = 0.0, v1 = 0.0, v2 = 0.0, v3 = 0.0;
-                if constexpr (sizeof(T) == 4) {
-                    LaneDotsF32 d;
+                LaneDotsF32 d;
 #pragma unroll
-                    for (int k = 0; k < RPL; ++k) {
-                        if (k >= rpl) break;
-                        d.add(x[k], y[k]);
-                    }
-                    v0 = d.a; v1 = d.b; v2 = d.gr; v3 = d.gi;
-                } else {
-#pragma unroll
-                    for (int k = 0; k < RPL; ++k) {
-                        if (k >= rpl) break;
-                        v0 += (double)x[k].x * x[k].x + (double)x[k].y * x[k].y;
-                        v1 += (double)y[k].x * y[k].x + (double)y[k].y * y[k].y;
-                        v2 += (double)x[k].x * y[k].x + (double)x[k].y * y[k].y;
-                        v3 += (double)x[k].x * y[k].y - (double)x[k].y * y[k].x;
-                    }
+                for (int k = 0; k < RPL; ++k) {
+                    if (k >= rpl) break;
+                    d.add(x[k], y[k]);
                 }
+                double v0 = d.a, v1 = d.b, v2 = d.gr, v3 = d.gi;
 #pragma unroll
                 for (int o = LPP / 2; o > 0; o >>= 1) {
                     v0 += __shfl_xor_sync(0xffffffffu, v0, o);
@@ -1211,8 +1201,8 @@ __device__ int lq_resident(double2* col, const int rc, const int R, const int N,
     return k < 1 ? 1 : k;
 }
 
-// One sweep-by-sweep circle-method Jacobi in shared memory with LPP lanes per pair (R <= 32 RPL / ...):
-// as jacobi_core, with the angle of jacobi_tau.
+// The complex128 Jacobi in shared memory, circle method, LPP lanes per pair (R <= LPP RPL), with the
+// angle of jacobi_tau.  (jacobi_core is complex64's.)
 template <int LPP, int RPL>
 __device__ void jacobi_core_d(double2* col, const int rc, const int R, const int N, const double tol,
                               const double tiny, const int max_sweeps, int* s_rot, int& sweeps, bool& converged,
