@@ -499,7 +499,7 @@ __device__ void svd_finish(const MpsView<T>& mps, const SvdWork<T>& wk, const Sv
     double* key = reinterpret_cast<double*>(smraw);  // [P2] then idx [P2]: 12 P2 bytes
     int* idx = reinterpret_cast<int*>(key + P2);
     for (int e = tid; e < P2; e += NT) {
-        key[e] = e < N ? wk.sig2[e] : -1.0;
+        key[e] = e < N ? fmax(wk.sig2[e], 0.0) : -1.0;  // (not a number counts as zero: padding stays last)
         idx[e] = e;
     }
     __syncthreads();
@@ -2089,6 +2089,8 @@ __device__ __forceinline__ void rc_stage(cplx_t<T>* dst, const cplx_t<T>* W, int
 }
 
 // descending bitonic sort of key[0..P2) carrying idx (ties: ascending idx); P2 a power of two
+// Keys descending, lower index first on ties.  Keys are numbers (a NaN would leave the order undefined and
+// let the padding's indices, beyond the columns, in among them).
 __device__ void bitonic_desc(double* key, int* idx, int P2) {
     const int tid = threadIdx.x, NT = blockDim.x;
     for (int k = 2; k <= P2; k <<= 1)
@@ -2223,7 +2225,7 @@ __device__ void svd_body_rc(const MpsView<T>& mps, const SvdWork<T>& wk, const S
                         sj += (double)w[row].x * w[row].x + (double)w[row].y * w[row].y;
                     sj = warp_sum(sj);
                 }
-                if (lane == 0) { key[c] = sj; idx[c] = c; }
+                if (lane == 0) { key[c] = c < N ? fmax(sj, 0.0) : sj; idx[c] = c; }
             }
             __syncthreads();
             bitonic_desc(key, idx, P2);
@@ -2572,7 +2574,7 @@ __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& 
             double* key = reinterpret_cast<double*>(smraw);
             int* idx = reinterpret_cast<int*>(key + P2);
             for (int c = tid; c < P2; c += NT) {
-                key[c] = c < N ? nrm[c] : -1.0;
+                key[c] = c < N ? fmax(nrm[c], 0.0) : -1.0;
                 idx[c] = c;
             }
             __syncthreads();
