@@ -964,6 +964,9 @@ private:
         for (auto& it : plan) *it.second = base_ + it.first;
         TQ_CK(cudaMemsetAsync(bar_, 0, sizeof(GridBar), stream_));
         TQ_CK(cudaMemsetAsync(stats_, 0, sizeof(RunStats), stream_));
+        // a Jacobi whose bounded waits ran out writes no column order, and what follows it reads one
+        TQ_CK(cudaMemsetAsync(perm_, 0, sizeof(int) * ld_, stream_));
+        TQ_CK(cudaMemsetAsync(sig_, 0, sizeof(double) * ld_, stream_));
         TQ_CK(cudaMemsetAsync(entropy_, 0, sizeof(double) * std::max(P_.steps, 1), stream_));
         TQ_CK(cudaMemsetAsync(envs_, 0, es * unit, stream_));  // the ONE env
         V one = mk<V>(1, 0);
