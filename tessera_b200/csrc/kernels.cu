@@ -675,7 +675,7 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
     constexpr int G = NT / BW;
     V* col = reinterpret_cast<V*>(smraw);  // [2*BW][rows_cap]
     __shared__ double red[4 * NW];         // [warps][4]
-    __shared__ int s_rot;
+    __shared__ int s_rot, s_ok;
     __shared__ __align__(8) uint64_t s_mbar;
     // complex128 in registers (D): squared norms of the staged columns, summed at the start of a sweep
     // (wk.sig2) and carried through each rotation, and which of the columns changed
@@ -756,33 +756,35 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                 // stage columns with 1-D TMA bulk copies: local c < BW -> block I, c >= BW -> block J
                 if (tid == 0) {
                     s_rot = 0;
-                    // the two blocks as their previous holders left them (the others then time out on
-                    // the copy below and leave too)
+                    // the two blocks as their previous holders left them, then the copies; one outcome of
+                    // both waits for the whole CTA
                     const int ver = sweep * (P - 1) + r;
-                    if (!flag_wait(&wk.flags[I], ver) || !flag_wait(&wk.flags[J], ver)) {
-                        atomicOr(status, ST_BARRIER_TIMEOUT);
-                        return;
+                    int ok = flag_wait(&wk.flags[I], ver) && flag_wait(&wk.flags[J], ver) ? 1 : 0;
+                    if (ok) {
+                        unsigned bytes = 0;
+                        for (int c = 0; c < 2 * BW; ++c) {
+                            const int gc = (c < BW) ? I * BW + c : J * BW + (c - BW);
+                            if (gc < N) bytes += (unsigned)(R * sizeof(V));
+                        }
+                        fence_proxy_async_global();
+                        mbar_expect_tx(&s_mbar, bytes);
+                        for (int c = 0; c < 2 * BW; ++c) {
+                            const int gc = (c < BW) ? I * BW + c : J * BW + (c - BW);
+                            if (gc < N)
+                                tma_load_1d(col + c * pp.rows_cap, W + (long long)gc * ld, (unsigned)(R * sizeof(V)),
+                                            &s_mbar);
+                        }
+                        if (!mbar_wait(&s_mbar, phase, 1000000000ull)) {
+                            ok = 0;
+                            mbar_wait(&s_mbar, phase, 1000000000ull);  // (bounded) for the copies in flight
+                        }
                     }
-                    unsigned bytes = 0;
-                    for (int c = 0; c < 2 * BW; ++c) {
-                        const int gc = (c < BW) ? I * BW + c : J * BW + (c - BW);
-                        if (gc < N) bytes += (unsigned)(R * sizeof(V));
-                    }
-                    fence_proxy_async_global();
-                    mbar_expect_tx(&s_mbar, bytes);
-                    for (int c = 0; c < 2 * BW; ++c) {
-                        const int gc = (c < BW) ? I * BW + c : J * BW + (c - BW);
-                        if (gc < N)
-                            tma_load_1d(col + c * pp.rows_cap, W + (long long)gc * ld, (unsigned)(R * sizeof(V)),
-                                        &s_mbar);
-                    }
+                    if (!ok) atomicOr(status, ST_BARRIER_TIMEOUT);
+                    s_ok = ok;
                 }
-                if (!mbar_wait(&s_mbar, phase, 1000000000ull)) {
-                    atomicOr(status, ST_BARRIER_TIMEOUT);
-                    // keep waiting (bounded) for the copies in flight before leaving
-                    mbar_wait(&s_mbar, phase, 1000000000ull);
-                    return;
-                }
+                __syncthreads();
+                if (!s_ok) return;
+                mbar_wait(&s_mbar, phase, 1000000000ull);  // complete: every thread sees the copies
                 phase ^= 1u;
                 int rot = 0;
                 if constexpr (D) {
