@@ -14,6 +14,22 @@ cudaError_t device_alloc(void** p, size_t bytes, bool pooled = false);
 void device_free(void* p);
 void device_trim();  // what the pool holds unused on the current device, back to the driver
 
+// Pooled memory of one call: on every way out, the work queued on the call's stream (null: the default
+// stream) is waited for before the memory goes back, since the pool may hand it to another thread at once.
+struct CallBuf {
+    char* p = nullptr;
+    cudaStream_t st;
+    explicit CallBuf(cudaStream_t s) : st(s) {}
+    CallBuf(const CallBuf&) = delete;
+    CallBuf& operator=(const CallBuf&) = delete;
+    ~CallBuf() {
+        if (!p) return;
+        cudaStreamSynchronize(st);
+        device_free(p);
+    }
+    cudaError_t alloc(size_t bytes) { return device_alloc((void**)&p, bytes, true); }
+};
+
 // ---------------------------------------------------------------------------------
 // Complex arithmetic on interleaved (re, im) pairs.  T = double (complex128 mode) or
 // float (complex64 mode).  Storage uses the CUDA vector types so loads are 16 / 8 byte

@@ -621,19 +621,12 @@ public:
         const MpsView<T> M = mps();
         ensure_obs();
         launch_chain<T>(M, 1, obsR_, n_, obs_, xs_, bar_, stats_, cap_, stream_);
-        int8_t* d = nullptr;
-        TQ_CK(device_alloc((void**)&d, count * (size_t)n_, true));
-        cudaError_t err = cudaSuccess;
-        try {
-            launch_sample<T>(M, obs_, (int)count, seed, d, stream_);
-        } catch (...) {
-            device_free(d);
-            throw;
-        }
-        err = cudaMemcpyAsync(spins, d, count * (size_t)n_, cudaMemcpyDeviceToHost, stream_);
-        if (err == cudaSuccess) err = cudaStreamSynchronize(stream_);
-        device_free(d);
-        TQ_CK(err);
+        CallBuf buf(stream_);
+        TQ_CK(buf.alloc(count * (size_t)n_));
+        int8_t* d = reinterpret_cast<int8_t*>(buf.p);
+        launch_sample<T>(M, obs_, (int)count, seed, d, stream_);
+        TQ_CK(cudaMemcpyAsync(spins, d, count * (size_t)n_, cudaMemcpyDeviceToHost, stream_));
+        TQ_CK(cudaStreamSynchronize(stream_));
         if (energies)
             for (size_t c = 0; c < count; ++c) {
                 const int8_t* x = spins + c * n_;
@@ -723,16 +716,8 @@ public:
     void svd_only(const double2* a, int R, int N, double* s, double2* u, double2* vh) {
         const int k = std::min(R, N);
         const size_t na = align256(sizeof(V) * (size_t)R * N), nu = align256(sizeof(V) * (size_t)R * k);
-        struct Buf {  // released on every way out
-            char* p = nullptr;
-            cudaStream_t st;
-            ~Buf() {
-                if (p) cudaStreamSynchronize(st);
-                device_free(p);
-            }
-        } buf;
-        buf.st = stream_;
-        TQ_CK(device_alloc((void**)&buf.p, na + nu + align256(sizeof(V) * (size_t)k * N), true));
+        CallBuf buf(stream_);
+        TQ_CK(buf.alloc(na + nu + align256(sizeof(V) * (size_t)k * N)));
         V* da = reinterpret_cast<V*>(buf.p);
         V* du = reinterpret_cast<V*>(buf.p + na);
         V* dv = reinterpret_cast<V*>(buf.p + na + nu);
@@ -1406,16 +1391,8 @@ public:
         const int B = (int)who.size();
         const size_t o_v = align256(sizeof(ObsTask<T>) * B), o_a = o_v + align256(sizeof(double) * ndots);
         const size_t o_s = o_a + align256(sizeof(double) * B);
-        struct Buf {  // released on every way out
-            char* p = nullptr;
-            cudaStream_t st;
-            ~Buf() {
-                if (p) cudaStreamSynchronize(st);
-                device_free(p);
-            }
-        } buf;
-        buf.st = st_;
-        TQ_CK(device_alloc((void**)&buf.p, o_s + align256(nspins), true));
+        CallBuf buf(st_);
+        TQ_CK(buf.alloc(o_s + align256(nspins)));
         ObsTask<T>* dt = reinterpret_cast<ObsTask<T>*>(buf.p);
         double *dv = reinterpret_cast<double*>(buf.p + o_v), *da = reinterpret_cast<double*>(buf.p + o_a);
         int8_t* ds = reinterpret_cast<int8_t*>(buf.p + o_s);

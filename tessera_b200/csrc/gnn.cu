@@ -32,11 +32,9 @@
 #include <vector>
 
 #include "../../include/tessera_qa.h"
+#include "common.cuh"
 
 namespace tq {
-
-cudaError_t device_alloc(void** p, size_t bytes, bool pooled = false);  // engine.cu: the library's pool, with failure injection
-void device_free(void* p);
 
 void set_last_error(const std::string& msg);
 
@@ -900,8 +898,9 @@ double tessera_qa_exact_ground(const double* h, size_t n, const size_t* ei, cons
         // and pattern
         const size_t o_w = al(8 * n), o_i = o_w + al(8 * m), o_j = o_i + al(4 * m), o_l = o_j + al(4 * m);
         const size_t o_d = o_l + 64, in_bytes = o_d + (scan ? 8 * n * n : 0), o_e = in_bytes, o_x = o_e + 8 * blocks, o_m = al(o_x + 8 * blocks);
-        char* arena = nullptr;
-        GN_CK(device_alloc((void**)&arena, o_m + al(8 * std::max<unsigned long long>(chunks, 1)), true));
+        CallBuf buf(nullptr);
+        GN_CK(buf.alloc(o_m + al(8 * std::max<unsigned long long>(chunks, 1))));
+        char* arena = buf.p;
         std::vector<char> up(in_bytes, (char)0xff), down(16 * blocks);
         std::memcpy(up.data(), h, 8 * n);
         if (m) {
@@ -939,7 +938,6 @@ double tessera_qa_exact_ground(const double* h, size_t n, const size_t* ei, cons
             err = cudaGetLastError();
         }
         if (err == cudaSuccess) err = cudaMemcpy(down.data(), be, 16 * blocks, cudaMemcpyDeviceToHost);
-        device_free(arena);
         GN_CK(err);
         const double* he = (const double*)down.data();
         const unsigned long long* hx = (const unsigned long long*)(down.data() + 8 * blocks);

@@ -533,21 +533,10 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         for (size_t i = 0; i < P->n; ++i)
             if (!std::isfinite(P->h[i])) throw std::invalid_argument("non-finite h");
         const unsigned long long dim = 1ull << n;
-        size_t freeb = 0, totb = 0;
-        SV_CK(cudaMemGetInfo(&freeb, &totb));
-        const size_t need = dim * (16 + 8 + 8) + (1 << 20);
-        if (need > freeb) {  // the library's own pool may hold some of it
-            device_trim();
-            SV_CK(cudaMemGetInfo(&freeb, &totb));
-        }
-        if (need > freeb) throw std::invalid_argument("not enough device memory for the 2^n state");
-        cudaStream_t st;
-        SV_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
         int nsm = 148, dev = 0;
         SV_CK(cudaGetDevice(&dev));
         SV_CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         const int grid = nsm * 8;
-        char* arena = nullptr;
         auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
         const bool tiled = n >= SV_TILE;
         const std::vector<SvPass> passes = tiled ? std::vector<SvPass>() : plan_passes(n);
@@ -564,7 +553,27 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         const size_t o_part = o_g + al((size_t)64 * n * made), o_ent = o_part + al(8 * (size_t)grid * (3 + SV_MAXN));
         const size_t o_bx = o_ent + al(8 * steps), o_rho = o_bx + al(8 * (size_t)grid);
         const size_t total = o_rho + al(32 * rho_blocks * held);
-        SV_CK(device_alloc((void**)&arena, total, true));
+        size_t freeb = 0, totb = 0;
+        SV_CK(cudaMemGetInfo(&freeb, &totb));
+        if (total > freeb) {  // the library's own pool may hold some of it
+            device_trim();
+            SV_CK(cudaMemGetInfo(&freeb, &totb));
+        }
+        if (total > freeb) throw std::invalid_argument("not enough device memory for the 2^n state");
+        struct Stream {  // the stream and the timing events, released on every way out
+            cudaStream_t st = nullptr;
+            cudaEvent_t e0 = nullptr, e1 = nullptr;
+            ~Stream() {
+                if (e0) cudaEventDestroy(e0);
+                if (e1) cudaEventDestroy(e1);
+                if (st) cudaStreamDestroy(st);
+            }
+        } own;
+        SV_CK(cudaStreamCreateWithFlags(&own.st, cudaStreamNonBlocking));
+        const cudaStream_t st = own.st;
+        CallBuf buf(st);
+        SV_CK(buf.alloc(total));
+        char* arena = buf.p;
         auto at = [&](size_t o) { return arena + o; };
         double2* psi = (double2*)at(o_psi);
         double *df = (double*)at(o_df), *dz = (double*)at(o_dz), *dh = (double*)at(o_h), *dw = (double*)at(o_w);
@@ -588,9 +597,8 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
             cp(dbias, P->bias, 8 * n);
             cp(dsc, P->schedule_c, 8 * steps);
         }
-        cudaEvent_t e0, e1;
-        if (err == cudaSuccess) err = cudaEventCreate(&e0);
-        if (err == cudaSuccess) err = cudaEventCreate(&e1);
+        if (err == cudaSuccess) err = cudaEventCreate(&own.e0);
+        if (err == cudaSuccess) err = cudaEventCreate(&own.e1);
         const size_t tile_bytes = tiled ? (sizeof(double2) << SV_TILE) / 16 * 17 : sizeof(double2) << passes[0].nt;
         if (err == cudaSuccess && tiled) {
             err = cudaFuncSetAttribute(k_sv_tile<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_bytes);
@@ -599,7 +607,7 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
         }
         if (err == cudaSuccess) err = cudaMemsetAsync(dent, 0, 8 * (size_t)steps, st);  // n = 1: no entanglement
         if (err == cudaSuccess) {
-            cudaEventRecord(e0, st);
+            cudaEventRecord(own.e0, st);
             k_sv_diag<<<grid, SV_NT, 0, st>>>(dh, di, dj, dw, n, m, dim, df, dz, psi);
             const SvPhase none{nullptr, 0.0};
             const double* hsb = P->schedule_b;
@@ -653,7 +661,7 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
                 }
             }
             k_sv_final<<<grid, SV_NT, 0, st>>>(psi, df, dim, n, part, dbx);
-            cudaEventRecord(e1, st);
+            cudaEventRecord(own.e1, st);
             err = cudaGetLastError();
         }
         std::vector<double> hp((size_t)grid * (3 + SV_MAXN));
@@ -666,11 +674,7 @@ extern "C" int tessera_qa_sv_anneal(const tessera_qa_problem* P, double dt, int 
             err = cudaMemcpyAsync(out->state, psi, dim * 16, cudaMemcpyDeviceToHost, st);
         if (err == cudaSuccess) err = cudaStreamSynchronize(st);
         float ms = 0;
-        if (err == cudaSuccess) cudaEventElapsedTime(&ms, e0, e1);
-        cudaEventDestroy(e0);
-        cudaEventDestroy(e1);
-        device_free(arena);
-        cudaStreamDestroy(st);
+        if (err == cudaSuccess) cudaEventElapsedTime(&ms, own.e0, own.e1);
         SV_CK(err);
         double tot = 0, ee = 0, bp = -1;
         unsigned long long bx = 0;
