@@ -796,7 +796,9 @@ private:
         add((void**)&du, sizeof(float) * (size_t)capN * H);
         add((void**)&da, sizeof(float) * (size_t)capN * H);
         add((void**)&dz, sizeof(float) * capN);
-        GN_CK(device_alloc((void**)&arena, off));
+        const cudaError_t err = device_alloc((void**)&arena, off);
+        if (err != cudaSuccess) capG = capN = capE = 0;  // no memory: nothing fits until a later call gets some
+        GN_CK(err);
         for (auto& it : plan) *it.second = static_cast<char*>(arena) + it.first;
     }
 };

@@ -47,3 +47,16 @@ def test_a_failed_allocation_ends_the_call_alone(lib):
         assert torch.cuda.mem_get_info()[0] == free0, name
         assert f() == want[name], name
     s.close()
+
+
+def test_a_network_that_could_not_grow_still_takes_a_smaller_batch(lib):
+    small, large = ([instances.dense_er(n, n, T=1.0, dt=0.1, chi=8) for n in ns] for ns in ((5, 6), (7, 8, 9, 10)))
+    net = learned.ScheduleGNN(hidden=16, layers=2, knots=8, seed=2)
+    want = net.forward(small)
+    lib.tessera_qa_debug_fail_allocations(0, 1)
+    with pytest.raises(_lib.EngineError) as err:
+        net.forward(large)
+    assert "out of memory" in str(err.value)
+    got = net.forward(small)
+    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    net.close()
