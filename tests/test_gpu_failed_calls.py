@@ -58,5 +58,6 @@ def test_a_network_that_could_not_grow_still_takes_a_smaller_batch(lib):
         net.forward(large)
     assert "out of memory" in str(err.value)
     got = net.forward(small)
-    assert all(np.array_equal(a, b) for a, b in zip(got, want))
+    for a, b in zip(got, want):  # the messages of a node are summed in no fixed order: a few FP32 roundings
+        np.testing.assert_allclose(a, b, rtol=1e-5, atol=1e-6)
     net.close()
