@@ -349,35 +349,21 @@ __device__ __forceinline__ bool jacobi_rotation(const double v0, const double v1
     return true;
 }
 
-__device__ __forceinline__ float sqrt_approx(const float x) {
-    float r;
-    asm("sqrt.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
-    return r;
-}
-
-// 1 / sqrt(x) for x in [1, 4): an FP32 start y (relative error 1e-7) and one third-order step
-// y (1 + e/2 + 3 e^2 / 8) with e = 1 - x y^2 of the series of (1 - e)^(-1/2), which leaves e^3
-__device__ __forceinline__ double rsqrt_near1(const double x) {
-    const double y = (double)rsqrtf((float)x);
-    const double e = fma(-x, y * y, 1.0);
-    return fma(y * e, fma(0.375, e, 0.5), y);
-}
-
-// tau = t e of the rotation w_p <- c (w_p - conj(tau) w_q), w_q <- c (w_q + tau w_p), from
-// alpha = |w_p|^2, beta = |w_q|^2, gamma = w_p^H w_q; false when the pair is converged or frozen.
-__device__ __forceinline__ bool jacobi_tau(const double a, const double b, const double gr, const double gi,
-                                           const double tol2, const double tiny, const bool mixed, double& tr,
-                                           double& ti) {
-    const double g2 = fma(gr, gr, gi * gi);
+// The rotation w_p <- c (w_p - conj(tau) w_q), w_q <- c (w_q + tau w_p), tau = s gamma, from alpha = |w_p|^2,
+// beta = |w_q|^2 and g2 = |gamma|^2, gamma = w_p^H w_q; false when the pair is converged or frozen.  FP64
+// throughout: with d = beta - alpha and h = sqrt(d^2 + 4 g2),
+//   c^2 = (1 + |d| / h) / 2,  s = 2 sgn(d) / (|d| + h) = sgn(d) / (h c^2),
+// so two rsqrt in turn give both; q = 1 / c.  c then takes a Newton step towards 1 / sqrt(1 + s^2 g2), which
+// makes the rotation unitary to rounding whatever the rounding of s.  The norms become alpha - s g2 and
+// beta + s g2.
+__device__ __forceinline__ bool jacobi_angle(const double a, const double b, const double g2, const double tol2,
+                                             const double tiny, const bool mixed, double& s, double& c, double& q) {
     if (!(pair_live(a, b, tiny, mixed) && g2 > tol2 * (a * b))) return false;
-    // 2^-exponent(max(a, b)): the scaled values fit FP32 (|gamma| >= 1e-13 sqrt(a b) >= 1e-30 max)
-    const int e = (__double2hiint(fmax(a, b)) >> 20) & 0x7ff;
-    const double f = __hiloint2double((2046 - e) << 20, 0);
-    const float d = (float)((b - a) * f), xr = (float)(gr * f), xi = (float)(gi * f);
-    const float h = sqrt_approx(fmaf(d, d, 4.f * fmaf(xr, xr, xi * xi)));
-    const float s = __fdividef(d >= 0.f ? 2.f : -2.f, fabsf(d) + h);
-    tr = (double)(xr * s);
-    ti = (double)(xi * s);
+    const double d = b - a, rh = rsqrt(fma(d, d, 4.0 * g2)), c2 = fma(0.5 * fabs(d), rh, 0.5);
+    q = rsqrt(c2);
+    s = copysign(rh * (q * q), d);
+    c = c2 * q;
+    c = fma(0.5 * c, fma(-c * c, fma(s, s * g2, 1.0), 1.0), c);
     return true;
 }
 
@@ -633,12 +619,13 @@ __device__ __forceinline__ int pair_tracked(double2* col, const int rc, const in
         x[k] = row < R ? col[p * rc + row] : make_double2(0.0, 0.0);
         y[k] = row < R ? col[q * rc + row] : make_double2(0.0, 0.0);
     }
-    double gr, gi, tr, ti;
+    double gr, gi, sn, c, rc1;
     const double a = nrm[p], b = nrm[q];
     lane_dot<RPL>(x, y, gr, gi);
     warp_sum2(gr, gi);
-    if (!jacobi_tau(a, b, gr, gi, tol * tol, tiny, mixed, tr, ti)) return 0;
-    const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2), cr = c * tr, ci = c * ti;
+    const double g2 = fma(gr, gr, gi * gi);
+    if (!jacobi_angle(a, b, g2, tol * tol, tiny, mixed, sn, c, rc1)) return 0;
+    const double cr = c * (sn * gr), ci = c * (sn * gi);
 #pragma unroll
     for (int k = 0; k < RPL; ++k) {
         const int row = lane + 32 * k;
@@ -649,9 +636,8 @@ __device__ __forceinline__ int pair_tracked(double2* col, const int rc, const in
         }
     }
     if (lane == 0) {
-        const double g = fma(tr, gr, ti * gi), c2 = c * c;
-        nrm[p] = fmax(0.0, c2 * fma(t2, b, fma(-2.0, g, a)));
-        nrm[q] = fmax(0.0, c2 * fma(t2, a, fma(2.0, g, b)));
+        nrm[p] = fmax(0.0, fma(-sn, g2, a));
+        nrm[q] = fmax(0.0, fma(sn, g2, b));
         chg[p] = 1;
         chg[q] = 1;
     }
@@ -856,13 +842,13 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                             yj[k] = (row < R) ? cq[row] : czero<V>();
                         }
                         if constexpr (D) {
-                            double gr, gi, tr, ti;
+                            double gr, gi, sn, c, rc1;
                             const double a = xn, b = *(volatile double*)&s_n[BW + q];
                             lane_dot<RPL>(xi, yj, gr, gi);
                             warp_sum2(gr, gi);
-                            if (ok && jacobi_tau(a, b, gr, gi, pp.tol * pp.tol, tiny, mixed, tr, ti)) {
-                                const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2);
-                                const double cr = c * tr, cim = c * ti;
+                            const double g2 = fma(gr, gr, gi * gi);
+                            if (ok && jacobi_angle(a, b, g2, pp.tol * pp.tol, tiny, mixed, sn, c, rc1)) {
+                                const double cr = c * (sn * gr), cim = c * (sn * gi);
 #pragma unroll
                                 for (int k = 0; k < RPL; ++k) {
                                     const int row = lane + 32 * k;
@@ -873,10 +859,9 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
                                                              fma(cim, u.x, fma(cr, u.y, c * v.y)));
                                     if (row < R) cq[row] = z;
                                 }
-                                const double g = fma(tr, gr, ti * gi), c2 = c * c;
-                                xn = fmax(0.0, c2 * fma(t2, b, fma(-2.0, g, a)));
+                                xn = fmax(0.0, fma(-sn, g2, a));
                                 if (lane == 0) {
-                                    s_n[BW + q] = fmax(0.0, c2 * fma(t2, a, fma(2.0, g, b)));
+                                    s_n[BW + q] = fmax(0.0, fma(sn, g2, b));
                                     s_c[BW + q] = 1;
                                     s_c[grp] = 1;
                                     ++rot;
@@ -1204,7 +1189,7 @@ __device__ int lq_resident(double2* col, const int rc, const int R, const int N,
 }
 
 // The complex128 Jacobi in shared memory, circle method, LPP lanes per pair (R <= LPP RPL), with the
-// angle of jacobi_tau.  (jacobi_core is complex64's.)
+// angle of jacobi_angle.  (jacobi_core is complex64's.)
 template <int LPP, int RPL>
 __device__ void jacobi_core_d(double2* col, const int rc, const int R, const int N, const double tol,
                               const double tiny, const int max_sweeps, int* s_rot, int& sweeps, bool& converged,
@@ -1260,11 +1245,9 @@ __device__ void jacobi_core_d(double2* col, const int rc, const int R, const int
                         gi += __shfl_xor_sync(0xffffffffu, gi, o);
                     }
                 }
-                double tr, ti;
-                if (ok && jacobi_tau(a, b, gr, gi, tol2, tiny, mixed, tr, ti)) {
-                    const double c = rsqrt_near1(fma(tr, tr, fma(ti, ti, 1.0)));
-                    tr *= c;
-                    ti *= c;
+                double sn, c, rc1;
+                if (ok && jacobi_angle(a, b, fma(gr, gr, gi * gi), tol2, tiny, mixed, sn, c, rc1)) {
+                    const double tr = c * (sn * gr), ti = c * (sn * gi);
 #pragma unroll
                     for (int k = 0; k < RPL; ++k) {
                         const double2 u = x[k], v = y[k];
@@ -2409,26 +2392,26 @@ __device__ void svd_body_rc(const MpsView<T>& mps, const SvdWork<T>& wk, const S
 //     X1' = X1 - conj(tau) (d_y / d_1) Y, Y' = Y + tau (d_1 / d_y) X1 with d scaled by c: 8
 //     multiply-adds per row instead of 12.  d falls by at most 1/sqrt(2) per rotation and is
 //     folded back into the columns at the start of each sweep (at most 511 rotations later).
-//   * The angle tau is formed in FP32 from FP64 inputs scaled by a power of two; c = 1 / sqrt(1 +
-//     |tau|^2) is FP64, so the rotation is unitary to FP64 whatever tau is, and an angle good to
-//     1e-7 leaves 1e-7 of gamma, which the next sweep takes with the rest.
+//   * Angles in FP64 with two rsqrt in turn each (jacobi_angle), so an annihilated inner product is zero to
+//     rounding and omega may go on as if it were; a first pair that was not rotated enters omega with its
+//     true inner product.
 //
 // Bound: the dots -> reduce -> angles -> update chain of a visit with two warps per scheduler (FP64
 // pipe 37 % busy: 12 multiply-adds per row and pair); shared memory moves 24 bytes per row and
-// pair.  148 graded 512 x 512 theta: 173 ms against 265 ms with one column per warp, three inner
-// products and unscaled rotations at the same 9.3 sweeps; 320 x 320: 65 against 94
-// ms.  Tried: y kept in registers
+// pair.  148 graded 512 x 512 theta: 177 ms against 265 ms with one column per warp, three inner
+// products and unscaled rotations at the same 9.4 sweeps; 320 x 320: 67 against 94 ms.  (Angles in FP32: 174
+// and 66 ms, and 1e-7 of every inner product left to the next sweep.)  Tried: y kept in registers
 // (183 ms, spills), no CTA barrier per J block but per-column hand-over (296 ms).
 // ------------------------------------------------------------------------------------
 constexpr int RCD_MAXN = 512;  // columns (2^-511 is the least a scale can reach within a sweep)
 
-// scale of a column (W = d X) and its reciprocal, after a rotation with cosine c: i = 1 / d kept to
+// scale of a column (W = d X) and its reciprocal, after a rotation with cosine c = 1 / q: i = 1 / d kept to
 // rounding by one Newton step
 struct ColScale {
     double d, i;
-    __device__ __forceinline__ void turn(const double c, const double t2) {
+    __device__ __forceinline__ void turn(const double c, const double q) {
         d *= c;
-        const double r = i * (c * (1.0 + t2));  // 1 / c = c (1 + t2)
+        const double r = i * q;
         i = r * fma(-d, r, 2.0);
     }
 };
@@ -2464,7 +2447,7 @@ __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& 
     __shared__ double nrm[RCD_MAXN];                           // |w|^2 by column
     __shared__ ColScale scl[RCD_MAXN];
     __shared__ int s_ver[JB];  // rounds each J slot has been through since the SVD began
-    __shared__ double s_ws[NW][8];
+    __shared__ double s_ws[NW][10];
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int R = pp.R > 0 ? pp.R : 2 * mps.dims[pp.bond];
     const int N0 = pp.N > 0 ? pp.N : 2 * mps.dims[pp.bond + 2];
@@ -2614,15 +2597,16 @@ __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& 
                             x[k] = buf[p * rc + row];
                             y[k] = buf[q * rc + row];
                         }
-                        double gr, gi, tr, ti;
+                        double gr, gi, sn, c, rc1;
                         lane_dot<RPL>(x, y, gr, gi);
                         warp_sum2(gr, gi);
                         ColScale sx = scl[cp], sy = scl[cq];
                         const double a = nrm[cp], b = nrm[cq], dd = sx.d * sy.d;
                         gr *= dd;
                         gi *= dd;
-                        if (jacobi_tau(a, b, gr, gi, tol2, tiny, mixed, tr, ti)) {
-                            const RotCoef rt(tr, ti, sx, sy);
+                        const double g2 = fma(gr, gr, gi * gi);
+                        if (jacobi_angle(a, b, g2, tol2, tiny, mixed, sn, c, rc1)) {
+                            const RotCoef rt(sn * gr, sn * gi, sx, sy);
 #pragma unroll
                             for (int k = 0; k < RPL; ++k) {
                                 const int row = lane + 32 * k;
@@ -2632,11 +2616,10 @@ __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& 
                                 buf[q * rc + row] = y[k];
                             }
                             if (lane == 0) {
-                                const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2), g = fma(tr, gr, ti * gi);
-                                nrm[cp] = fmax(0.0, c * c * fma(t2, b, fma(-2.0, g, a)));
-                                nrm[cq] = fmax(0.0, c * c * fma(t2, a, fma(2.0, g, b)));
-                                sx.turn(c, t2);
-                                sy.turn(c, t2);
+                                nrm[cp] = fmax(0.0, fma(-sn, g2, a));
+                                nrm[cq] = fmax(0.0, fma(sn, g2, b));
+                                sx.turn(c, rc1);
+                                sy.turn(c, rc1);
                                 scl[cp] = sx;
                                 scl[cq] = sy;
                                 ++rot;
@@ -2734,29 +2717,30 @@ __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& 
                     g2i *= d2;
                     // both angles first, then one pass over the rows for both rotations
                     RotCoef q1, q2;
-                    double tr, ti, cc1 = 1.0, tt1 = 0.0;
-                    const bool t1 = jacobi_tau(a1, ay, g1r, g1i, tol2, tiny, mixed, tr, ti);
+                    double sn1, sn2, cc1 = 1.0, cc2, rc1, rc2, gg1 = fma(g1r, g1r, g1i * g1i);
+                    const bool t1 = jacobi_angle(a1, ay, gg1, tol2, tiny, mixed, sn1, cc1, rc1);
                     if (t1) {
-                        const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2);
-                        const double g = fma(tr, g1r, ti * g1i), c2 = c * c;
+                        const double tr = sn1 * g1r, ti = sn1 * g1i;
                         q1 = RotCoef(tr, ti, s1, sy);
-                        const double an = fmax(0.0, c2 * fma(t2, ay, fma(-2.0, g, a1)));
-                        ay = fmax(0.0, c2 * fma(t2, a1, fma(2.0, g, ay)));
-                        a1 = an;
-                        sy.turn(c, t2);
+                        a1 = fmax(0.0, fma(-sn1, gg1, a1));
+                        ay = fmax(0.0, fma(sn1, gg1, ay));
+                        sy.turn(cc1, rc1);
                         // gamma2 = c (gamma2 + tau omega), omega = c (omega - conj(tau) gamma2)
-                        const double nr = c * fma(-ti, wi, fma(tr, wr, g2r));
-                        const double ni = c * fma(ti, wr, fma(tr, wi, g2i));
-                        wr = c * fma(-ti, g2i, fma(-tr, g2r, wr));
-                        wi = c * fma(ti, g2r, fma(-tr, g2i, wi));
+                        const double nr = cc1 * fma(-ti, wi, fma(tr, wr, g2r));
+                        const double ni = cc1 * fma(ti, wr, fma(tr, wi, g2i));
+                        wr = cc1 * fma(-ti, g2i, fma(-tr, g2r, wr));
+                        wi = cc1 * fma(ti, g2r, fma(-tr, g2i, wi));
                         g2r = nr;
                         g2i = ni;
-                        cc1 = c;
-                        tt1 = t2;
                         if (lane == 0) ++rot;
                     }
-                    const bool t2nd = jacobi_tau(a2, ay, g2r, g2i, tol2, tiny, mixed, tr, ti);
-                    if (t2nd) q2 = RotCoef(tr, ti, s2, sy);
+                    if (lane == 0) {  // w_1^H y as the first rotation, if any, left it
+                        ws[8] = t1 ? 0.0 : g1r;
+                        ws[9] = t1 ? 0.0 : g1i;
+                    }
+                    const double gg2 = fma(g2r, g2r, g2i * g2i);
+                    const bool t2nd = jacobi_angle(a2, ay, gg2, tol2, tiny, mixed, sn2, cc2, rc2);
+                    if (t2nd) q2 = RotCoef(sn2 * g2r, sn2 * g2i, s2, sy);
                     if (t1 || t2nd) {
 #pragma unroll
                         for (int k = 0; k < RPL; ++k) {
@@ -2766,18 +2750,18 @@ __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& 
                             q2.apply(x2[k], v, zo, v);
                             cq[32 * k] = v;
                         }
-                        if (t1) s1.turn(cc1, tt1);
+                        if (t1) s1.turn(cc1, rc1);
                         if (t2nd) {
-                            const double t2 = fma(tr, tr, ti * ti), c = rsqrt_near1(1.0 + t2);
-                            const double g = fma(tr, g2r, ti * g2i), c2 = c * c;
-                            const double an = fmax(0.0, c2 * fma(t2, ay, fma(-2.0, g, a2)));
-                            ay = fmax(0.0, c2 * fma(t2, a2, fma(2.0, g, ay)));
-                            a2 = an;
-                            s2.turn(c, t2);
-                            sy.turn(c, t2);
-                            wr *= c;  // x1^H y' was just annihilated
-                            wi *= c;
-                            if (lane == 0) ++rot;
+                            a2 = fmax(0.0, fma(-sn2, gg2, a2));
+                            ay = fmax(0.0, fma(sn2, gg2, ay));
+                            s2.turn(cc2, rc2);
+                            sy.turn(cc2, rc2);
+                            if (lane == 0) {  // omega = c (omega - tau conj(gamma1))
+                                const double tr = sn2 * g2r, ti = sn2 * g2i, hr = ws[8], hi = ws[9];
+                                wr = cc2 * fma(-ti, hi, fma(-tr, hr, wr));
+                                wi = cc2 * fma(tr, hi, fma(-ti, hr, wi));
+                                ++rot;
+                            }
                         }
                         if (lane == 0) {
                             *(volatile double*)&nrm[cy] = ay;
