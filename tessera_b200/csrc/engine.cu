@@ -724,7 +724,7 @@ public:
         TQ_CK(cudaMemcpyAsync(da, a, sizeof(V) * (size_t)R * N, cudaMemcpyHostToDevice, stream_));
         launch_svd_load<T>(da, R, N, W_, ld_, stream_);
         const int bw = pick_block(R, N);
-        launch_svd<T>(mps(), 0, k, tol_for(R), C_.max_sweeps, work(), R, N, bw, stream_, R, N);
+        launch_svd<T>(mps(), 0, k, tol_for(R, false), C_.max_sweeps, work(), R, N, bw, stream_, R, N);
         if (u || vh) launch_svd_u<T>(W_, ld_, perm_, sig_, R, k, du, stream_);
         std::vector<double> sg(k);
         RunStats st;
@@ -765,7 +765,9 @@ public:
         t.pp.N = 0;
         t.pp.no_trunc = 0;
         t.pp.chi = C_.chi;
-        t.pp.tol = tol_for(2 * cap_);
+        // (the batched LQ runs before every Jacobi but the block-Gram one; the resident one has its own)
+        const bool lq = C_.precond != 2 && (C_.block != 32 || svd_resident<T>(2 * cap_, 2 * cap_));
+        t.pp.tol = tol_for(2 * cap_, lq && cap_ <= 128);
         t.pp.tiny = sizeof(T) == 8 ? 1e-200 : 1e-60;
         t.pp.max_sweeps = C_.max_sweeps;
         t.pp.rows_cap = rows_cap;
@@ -854,13 +856,17 @@ private:
     }
     SvdWork<T> work() const { return SvdWork<T>{theta_, W_, ld_, sig2_, sig_, perm_, counters_, scal_, bar_, stats_, flags_}; }
 
-    double tol_for(int R) const {
+    // fine: the Jacobi works on an LQ factor.  Its leftover inner products lean one way, and an anneal's norm
+    // drifts with them: over 660 updates of n = 12, chi = 64 by 7.9e-12 (rms) at 1e-13 against 6.2e-12 without
+    // the LQ, by 1.5e-12 at 2e-14, for under 2% of time (9.0 sweeps instead of 8.9).  A batch above 256 rows,
+    // which has always had the LQ, stays at 1e-13 (2e-14 would cost it 9.8 sweeps instead of 9.4).
+    double tol_for(int R, bool fine) const {
         if (C_.tol > 0) return C_.tol;
         const double eps = sizeof(T) == 8 ? 2.220446049250313e-16 : 1.1920928955078125e-07;
         // stop rotating a pair once |w_p^H w_q| <= tol |w_p||w_q|: 1e-13 in complex128 (a few
         // hundred ulps above the rounding floor of the FP64 dot products), 8 sqrt(R) ulps of
         // float in complex64 (whose dot products are accumulated in FP64)
-        return sizeof(T) == 8 ? std::max(1e-13, 4.0 * std::sqrt((double)R) * eps)
+        return sizeof(T) == 8 ? std::max(fine ? 2e-14 : 1e-13, 4.0 * std::sqrt((double)R) * eps)
                               : 8.0 * std::sqrt((double)std::max(R, 16)) * eps;
     }
 
@@ -1068,8 +1074,9 @@ private:
             b = event();
             TQ_CK(cudaEventRecord(a, stream_));
         }
-        launch_svd<T>(M, i, C_.chi, tol_for(2 * dl), C_.max_sweeps, work(), 2 * dl, 2 * dr, pick_block(2 * dl, 2 * dr),
-                      stream_, 0, 0, lq ? 1 : 0, C_.precond != 2 ? 1 : 0);
+        launch_svd<T>(M, i, C_.chi, tol_for(2 * dl, lq || (C_.precond != 2 && !wide)), C_.max_sweeps, work(),
+                      2 * dl, 2 * dr, pick_block(2 * dl, 2 * dr), stream_, 0, 0, lq ? 1 : 0,
+                      C_.precond != 2 ? 1 : 0);
         if (C_.timing) {
             TQ_CK(cudaEventRecord(b, stream_));
             timed_.push_back({a, b});
