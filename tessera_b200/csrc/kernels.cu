@@ -968,8 +968,9 @@ __device__ __forceinline__ void svd_body(const MpsView<T>& mps, const SvdWork<T>
 // disjoint pairs.  A pair is owned by LPP lanes (RPL complex rows per lane, R <= LPP RPL),
 // so a warp rotates 32/LPP pairs at once and the reduction is log2(LPP) shuffle levels.
 // A sweep is N-1 rounds; a sweep without a rotation ends the iteration.  LPP by size class:
-// 8 up to R = 64, 16 up to 128, 32 up to 256.  One instantiation serves a whole class, so a
-// theta is rotated by the same instructions whatever batch it runs in.
+// 8 up to R = 64, 16 up to 128, 32 up to 256, in complex128 with the choice of resident_jacobi.
+// Lanes follow from the theta and its launch's class, so a theta is rotated by the same
+// instructions alone and in any batch of that class.
 // complex64 (jacobi_core): up to 8 register rows per lane; alpha, beta, gamma are FP32 lane sums
 // reduced in FP64 and the rotation is jacobi_rotation's.  complex128: lq_resident, then
 // jacobi_core_d over its rank.
@@ -1281,8 +1282,11 @@ __device__ void jacobi_core_d(double2* col, const int rc, const int R, const int
 }
 
 // The resident Jacobi of a class (LPP lanes per pair hold its rows): complex64 always with LPP
-// lanes; complex128 with more lanes a pair where that still takes every pair in one turn, since a
-// round then lasts as long as one pair's chain (loads, products, reduction, angle, update).
+// lanes; complex128 with more lanes a pair where 256 threads, which every resident launch has, still take
+// every pair in one turn, since a round then lasts as long as one pair's chain (loads, products, reduction,
+// angle, update).  Lanes, and so the order of the sums, follow from the theta and its class alone, not from
+// the launch's threads: a theta comes out the same bits alone and in a batch of its class.
+constexpr int RES_LANES = 256;
 template <typename T, int LPP>
 __device__ __forceinline__ void resident_jacobi(cplx_t<T>* col, const int rc, const int R, const int N,
                                                 const double tol, const double tiny, const int max_sweeps, int* s_rot,
@@ -1290,10 +1294,10 @@ __device__ __forceinline__ void resident_jacobi(cplx_t<T>* col, const int rc, co
     if constexpr (sizeof(T) == 4) {
         jacobi_core<T, LPP>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
     } else {
-        const int npairs = (N + 1) / 2, NT = blockDim.x;
-        if (npairs * 32 <= NT)
+        const int npairs = (N + 1) / 2;
+        if (npairs * 32 <= RES_LANES)
             jacobi_core_d<32, LPP / 4>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
-        else if (LPP <= 16 && npairs * 16 <= NT)
+        else if (LPP <= 16 && npairs * 16 <= RES_LANES)
             jacobi_core_d<16, LPP / 2>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
         else
             jacobi_core_d<LPP, 8>(col, rc, R, N, tol, tiny, max_sweeps, s_rot, sweeps, converged, rotations);
