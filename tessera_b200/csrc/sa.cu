@@ -10,21 +10,28 @@
 // splitmix64 stream keyed by (seed, instance, restart, sweep, spin), so a run is reproducible
 // and the CPU oracle restates it draw for draw.
 //
-// Layout: SA_G lanes per restart chain, as many CTAs per instance as it takes to fill the GPU (each
+// Layout: 8 lanes per restart chain, as many CTAs per instance as it takes to fill the GPU (each
 // strides over the instance's restarts); the last CTA of an instance to finish picks the winner.
-// The coupling graph sits in shared memory as adjacency lists (offsets, neighbour, weight; repeated
-// pairs merged); a chain's spins are a bit mask of SA_MAXN bits in registers (bit i set <-> s_i =
-// -1), and its local fields h_i + sum_j J_ij s_j are kept in shared memory and changed only where a
-// flip changes them, the chain's lanes sharing the neighbours.  A visit that does not flip, the
-// usual one once the chain has cooled, costs no walk over the neighbours.  Each lane draws the
-// uniform of every SA_G-th spin and the temperature of every SA_G-th sweep, and shuffles hand them
-// round.  The Metropolis test is decided in FP32 where FP32 can tell, u outside (1 -+ 1e-4) exp(-dE
-// / t), and by the FP64 exp otherwise, so every decision is the FP64 one.
+// The coupling graph sits in shared memory as adjacency lists (offsets, neighbour, weight, in the
+// order of the edge list); a chain's spins are a bit mask of SA_MAXN bits in registers (bit i set <->
+// s_i = -1), and its local fields h_i + sum_j J_ij s_j are kept in shared memory and changed only
+// where a flip changes them, the chain's lanes sharing the neighbours (one lane takes them all where
+// a pair is repeated).  A visit that does not flip, the usual one once the chain has cooled, costs no
+// walk over the neighbours.  Each lane draws the uniform of every 8th spin and the temperature of
+// every 8th sweep, and shuffles hand them round.
+//
+// A decision rests on the kept field and FP32 only where these can tell: u outside (1 -+ 1e-4) exp(-dE
+// / t).  Of that margin __expf and the rounding of its argument take 1.2e-5 (for arguments up to 37,
+// beyond which no u but 0 is as small) and the kept field at most 1e-5: fields are summed afresh every
+// SA_FRESH sweeps, a task carries a bound on what rounding can do to them in between, and a sweep at a
+// temperature for which that is not enough (or out of FP32's range) takes no decision this way.  All
+// others are the FP64 test on the field summed there and then, neighbours in the edge list's order, so
+// every decision is that test's.
 //
 // Bound: the latency of a visit (shuffle, field, test, a flip's walk).  8 dense n = 48 instances,
 // 512 restarts x 500 sweeps: 84 ms with one thread per chain, 128 chains a CTA and the field summed
 // at every visit; 20.5 ms with one CTA per 32 chains and kept fields (a warp then walks at nearly
-// every visit, for whichever chain flips); 6.4 ms with 8 lanes per chain.
+// every visit, for whichever chain flips); 5.4 ms with 8 lanes per chain.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -44,6 +51,7 @@ constexpr int SA_WORDS = SA_MAXN / 64;
 constexpr int SA_G = 8;            // lanes per chain
 constexpr int SA_THREADS = 128;
 constexpr int SA_CHAINS = SA_THREADS / SA_G;  // 16: their fields (16 KB at 128 spins) fit beside any graph
+constexpr int SA_FRESH = 64;       // sweeps between fresh sums of the kept fields
 constexpr int SA_CTAS_PER_SM = 8;  // CTAs to aim at before a CTA takes more than one turn of restarts
 
 #define SA_CK(x)                                                                                          \
@@ -68,6 +76,8 @@ struct SaTask {
     int hoff;  // first field / spin of this instance
     int eoff;  // first edge of this instance
     int m;     // its edges (self-loops included: they enter the energy)
+    int rep;   // 1: some pair of spins is coupled more than once
+    double err;  // bound on what rounding makes of an energy change taken from the kept fields
 };
 
 // best chain of one CTA
@@ -116,20 +126,24 @@ __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const in
         unsigned long long bits[SA_WORDS] = {};
         for (int i = 0; i < n; ++i)  // random start: s_i = -1 with probability 1/2
             if (sa_uniform(seed, blockIdx.x, r, sweeps, i, sweeps, n) < 0.5) bits[i >> 6] |= 1ull << (i & 63);
-        for (int i = gl; i < n; i += SA_G) {
+        auto field = [&](int i) {
             double f = sh[i];
             for (int e = so[i]; e < so[i + 1]; ++e) {
                 const int j = sn[e];
                 f += ((bits[j >> 6] >> (j & 63)) & 1ull) ? -sw[e] : sw[e];
             }
-            fld[i] = f;
-        }
-        __syncwarp();
+            return f;
+        };
         double tl = 0.0;
         for (int k = 0; k < sweeps; ++k) {
+            if (k % SA_FRESH == 0) {
+                for (int i = gl; i < n; i += SA_G) fld[i] = field(i);
+                __syncwarp();
+            }
             if (k % SA_G == 0) tl = t0 * pow(ratio, (double)(k + gl) / den);
             const double t = __shfl_sync(0xffffffffu, tl, k % SA_G, SA_G);
             const float it = (float)(1.0 / t);
+            const bool quick = t > 1e-30 && t < 1e30 && tk.err < 1e-5 * t;
             for (int i0 = 0; i0 < n; i0 += SA_G) {
                 const double ul = sa_uniform(seed, blockIdx.x, r, k, i0 + gl, sweeps, n);
                 const int i1 = n - i0 < SA_G ? n - i0 : SA_G;
@@ -137,18 +151,17 @@ __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const in
                     const int i = i0 + s;
                     const double u = __shfl_sync(0xffffffffu, ul, s, SA_G);
                     const bool neg = (bits[i >> 6] >> (i & 63)) & 1ull;
-                    const double f = fld[i];
-                    const double de = 2.0 * (neg ? -f : f);
-                    bool flip = de < 0.0;
-                    if (!flip) {
-                        const float p = __expf(-(float)de * it), v = (float)u;
-                        if (v < p * 0.9999f) flip = true;
-                        else if (!(v > p * 1.0001f) || v == 0.f) flip = u < exp(-de / t);  // FP32 cannot tell
+                    const double fk = fld[i];
+                    const float p = __expf((float)(neg ? fk : -fk) * 2.f * it), v = (float)u;
+                    bool flip = v < p * 0.9999f;
+                    if (!quick || (!flip && (!(v > p * 1.0001f) || v == 0.f))) {
+                        const double f = field(i), de = 2.0 * (neg ? -f : f);
+                        flip = de < 0.0 || u < exp(-de / t);
                     }
                     if (flip) {
                         bits[i >> 6] ^= 1ull << (i & 63);
-                        const int e1 = so[i + 1];
-                        for (int e = so[i] + gl; e < e1; e += SA_G) {  // s_i changed by +2 if it was -1, else -2
+                        const int e1 = so[i + 1], step = tk.rep ? 1 : SA_G;
+                        for (int e = tk.rep && gl ? e1 : so[i] + gl; e < e1; e += step) {  // s_i: +2 if it was -1, else -2
                             const double w2 = 2.0 * sw[e];
                             fld[sn[e]] += neg ? w2 : -w2;
                         }
@@ -227,7 +240,7 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
         // given (self-loops included, as Ising::energy does); the dynamics skip self-loops,
         // which only add a constant.
         std::vector<SaTask> tasks(count);
-        std::vector<int> where;  // (spin, spin) -> its place in the first spin's list
+        std::vector<char> seen;  // (spin, spin): coupled already
         std::vector<int> adj_off, nbr, ei, ej;
         std::vector<double> w, h, ew;
         size_t smem = 0;
@@ -238,11 +251,10 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
                                             std::to_string(SA_MAXN) + " and non-NULL arrays");
             const int n = (int)p.n;
             std::vector<std::vector<std::pair<int, double>>> adj(n);
-            where.assign(p.n * p.n, -1);
-            size_t listed = 0;  // entries as given, repeated pairs and all: what the size limit counts
+            seen.assign(p.n * p.n, 0);
             for (int i = 0; i < n; ++i)
                 if (!std::isfinite(p.h[i])) throw std::invalid_argument("non-finite field");
-            SaTask t{n, (int)h.size(), (int)ei.size(), (int)p.m};
+            SaTask t{n, (int)h.size(), (int)ei.size(), (int)p.m, 0, 0.0};
             for (size_t e = 0; e < p.m; ++e) {
                 const size_t i = p.ei[e], j = p.ej[e];
                 if (i >= p.n || j >= p.n || !std::isfinite(p.ew[e]))
@@ -251,29 +263,29 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
                 ej.push_back((int)j);
                 ew.push_back(p.ew[e]);
                 if (i == j) continue;
-                listed += 2;
-                for (int side = 0; side < 2; ++side) {  // a repeated pair adds to its first entry
-                    auto& row = adj[side ? j : i];
-                    const int other = (int)(side ? i : j);
-                    int& at = where[(side ? j : i) * p.n + other];
-                    if (at < 0) {
-                        at = (int)row.size();
-                        row.push_back({other, p.ew[e]});
-                    } else {
-                        row[at].second += p.ew[e];
-                    }
-                }
+                adj[i].push_back({(int)j, p.ew[e]});
+                adj[j].push_back({(int)i, p.ew[e]});
+                if (seen[i * p.n + j]) t.rep = 1;
+                seen[i * p.n + j] = seen[j * p.n + i] = 1;
             }
+            size_t deg = 0;
             for (int i = 0; i < n; ++i) {
                 h.push_back(p.h[i]);
                 adj_off.push_back((int)nbr.size());
+                double span = std::fabs(p.h[i]);
                 for (auto& pr : adj[i]) {
                     nbr.push_back(pr.first);
                     w.push_back(pr.second);
+                    span += std::fabs(pr.second);
                 }
+                // half an ulp of at most `span` per term: SA_FRESH sweeps in which every neighbour flips, the
+                // fresh sum before them and the one the decision stands for; an energy change is twice that
+                const double d = (double)adj[i].size();
+                t.err = std::max(t.err, 2.0 * 0x1p-53 * span * ((SA_FRESH + 2) * d + 8.0));
+                deg += adj[i].size();
             }
             tasks[b] = t;
-            smem = std::max(smem, listed * (sizeof(double) + sizeof(short)) + n * sizeof(double) +
+            smem = std::max(smem, deg * (sizeof(double) + sizeof(short)) + n * sizeof(double) +
                                       (n + 1) * sizeof(int) + 64);
         }
         adj_off.push_back((int)nbr.size());
