@@ -10,15 +10,16 @@
 // splitmix64 stream keyed by (seed, instance, restart, sweep, spin), so a run is reproducible
 // and the CPU oracle restates it draw for draw.
 //
-// Layout: 8 lanes per restart chain, as many CTAs per instance as it takes to fill the GPU (each
+// Layout: 8, 4 or 1 lanes per restart chain (tessera_qa_sa_solve chooses), as many CTAs per instance as it takes to fill the GPU (each
 // strides over the instance's restarts); the last CTA of an instance to finish picks the winner.
 // The coupling graph sits in shared memory as adjacency lists (offsets, neighbour, weight, in the
 // order of the edge list); a chain's spins are a bit mask of SA_MAXN bits in registers (bit i set <->
 // s_i = -1), and its local fields h_i + sum_j J_ij s_j are kept in shared memory and changed only
 // where a flip changes them, the chain's lanes sharing the neighbours (one lane takes them all where
 // a pair is repeated).  A visit that does not flip, the usual one once the chain has cooled, costs no
-// walk over the neighbours.  Each lane draws the uniform of every 8th spin and the temperature of
-// every 8th sweep, and shuffles hand them round.
+// walk over the neighbours.  With G lanes, each draws the uniform of every G-th spin and the
+// temperature of every G-th sweep, and shuffles hand them round.  (Without kept fields, KEEP false, a
+// field is summed at each visit.)
 //
 // A decision rests on the kept field and FP32 only where these can tell: u outside (1 -+ 1e-4) exp(-dE
 // / t).  Of that margin __expf and the rounding of its argument take 1.2e-5 (for arguments up to 37,
@@ -48,9 +49,7 @@ namespace tq {
 
 constexpr int SA_MAXN = 128;
 constexpr int SA_WORDS = SA_MAXN / 64;
-constexpr int SA_G = 8;            // lanes per chain
 constexpr int SA_THREADS = 128;
-constexpr int SA_CHAINS = SA_THREADS / SA_G;  // 16: their fields (16 KB at 128 spins) fit beside any graph
 constexpr int SA_FRESH = 64;       // sweeps between fresh sums of the kept fields
 constexpr int SA_CTAS_PER_SM = 8;  // CTAs to aim at before a CTA takes more than one turn of restarts
 
@@ -94,21 +93,24 @@ __device__ __forceinline__ bool sa_before(const double e, const int r, const dou
     return e < e2 || (e == e2 && r < r2);
 }
 
+template <int SA_G, bool KEEP>
 __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const int* adj_off, const int* adj_nbr,
                                                    const double* adj_w, const double* h, const int* ei, const int* ej,
                                                    const double* ew, int restarts, int sweeps, double t0,
                                                    double t_end, unsigned long long seed, SaBest* part, int* tickets,
                                                    double* out_e, int8_t* out_s) {
+    constexpr int SA_CHAINS = SA_THREADS / SA_G;
     extern __shared__ __align__(16) unsigned char smraw[];
     const SaTask tk = tasks[blockIdx.x];
     const int tid = threadIdx.x, chain = tid / SA_G, gl = tid % SA_G;
     const int n = tk.n, a0 = adj_off[tk.hoff], deg_tot = adj_off[tk.hoff + n] - a0;
     double* fld = reinterpret_cast<double*>(smraw) + chain * n;      // [n] this chain's local fields
-    double* sw = reinterpret_cast<double*>(smraw) + SA_CHAINS * n;   // [deg_tot] weights
+    double* sw = reinterpret_cast<double*>(smraw) + (KEEP ? SA_CHAINS * n : 0);  // [deg_tot] weights
     double* sh = sw + deg_tot;                                       // [n] fields
     int* so = reinterpret_cast<int*>(sh + n);                        // [n + 1] offsets
     short* sn = reinterpret_cast<short*>(so + n + 1);                // [deg_tot] neighbours
     __shared__ SaBest s_best[SA_CHAINS];
+    __shared__ unsigned long long s_bits[SA_CHAINS][SA_WORDS];
     __shared__ int s_last;
     for (int e = tid; e < deg_tot; e += SA_THREADS) {
         sw[e] = adj_w[a0 + e];
@@ -120,12 +122,15 @@ __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const in
     const double ratio = t_end / t0;
     const double den = (double)((sweeps < 2 ? 2 : sweeps) - 1);
     SaBest best{INFINITY, -1, 0, {}};
-    // every lane of a warp takes the same turns (a chain past the last restart runs along unseen)
+    // every thread of the CTA takes the same turns (a chain past the last restart runs along unseen)
     for (int r0 = blockIdx.y * SA_CHAINS; r0 < restarts; r0 += gridDim.y * SA_CHAINS) {
         const int r = r0 + chain;
         unsigned long long bits[SA_WORDS] = {};
-        for (int i = 0; i < n; ++i)  // random start: s_i = -1 with probability 1/2
+        for (int i = gl; i < n; i += SA_G)  // random start: s_i = -1 with probability 1/2
             if (sa_uniform(seed, blockIdx.x, r, sweeps, i, sweeps, n) < 0.5) bits[i >> 6] |= 1ull << (i & 63);
+#pragma unroll
+        for (int o = SA_G / 2; o > 0; o >>= 1)
+            for (int w = 0; w < SA_WORDS; ++w) bits[w] |= __shfl_xor_sync(0xffffffffu, bits[w], o, SA_G);
         auto field = [&](int i) {
             double f = sh[i];
             for (int e = so[i]; e < so[i + 1]; ++e) {
@@ -136,7 +141,7 @@ __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const in
         };
         double tl = 0.0;
         for (int k = 0; k < sweeps; ++k) {
-            if (k % SA_FRESH == 0) {
+            if (KEEP && k % SA_FRESH == 0) {
                 for (int i = gl; i < n; i += SA_G) fld[i] = field(i);
                 __syncwarp();
             }
@@ -151,17 +156,17 @@ __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const in
                     const int i = i0 + s;
                     const double u = __shfl_sync(0xffffffffu, ul, s, SA_G);
                     const bool neg = (bits[i >> 6] >> (i & 63)) & 1ull;
-                    const double fk = fld[i];
+                    const double fk = KEEP ? fld[i] : field(i);
                     const float p = __expf((float)(neg ? fk : -fk) * 2.f * it), v = (float)u;
                     bool flip = v < p * 0.9999f;
                     if (!quick || (!flip && (!(v > p * 1.0001f) || v == 0.f))) {
-                        const double f = field(i), de = 2.0 * (neg ? -f : f);
+                        const double f = KEEP ? field(i) : fk, de = 2.0 * (neg ? -f : f);
                         flip = de < 0.0 || u < exp(-de / t);
                     }
                     if (flip) {
                         bits[i >> 6] ^= 1ull << (i & 63);
-                        const int e1 = so[i + 1], step = tk.rep ? 1 : SA_G;
-                        for (int e = tk.rep && gl ? e1 : so[i] + gl; e < e1; e += step) {  // s_i: +2 if it was -1, else -2
+                        const int e1 = KEEP ? so[i + 1] : 0, step = tk.rep ? 1 : SA_G;
+                        for (int e = !KEEP || (tk.rep && gl) ? e1 : so[i] + gl; e < e1; e += step) {  // s_i: +2 if it was -1, else -2
                             const double w2 = 2.0 * sw[e];
                             fld[sn[e]] += neg ? w2 : -w2;
                         }
@@ -170,21 +175,27 @@ __global__ void __launch_bounds__(SA_THREADS) k_sa(const SaTask* tasks, const in
                 }
             }
         }
-        double en = 0.0;  // E = -sum w s_i s_j - sum h s_i, in the order of the edge list
-        for (int e = 0; e < tk.m; ++e) {
-            const int i = ei[tk.eoff + e], j = ej[tk.eoff + e];
-            const bool si = (bits[i >> 6] >> (i & 63)) & 1ull, sj = (bits[j >> 6] >> (j & 63)) & 1ull;
-            en -= (si == sj) ? ew[tk.eoff + e] : -ew[tk.eoff + e];
+        if (gl == 0)
+            for (int w = 0; w < SA_WORDS; ++w) s_bits[chain][w] = bits[w];
+        __syncthreads();
+        if (tid < SA_CHAINS) {  // one thread a chain: E = -sum w s_i s_j - sum h s_i, in the order of the edge list
+            const unsigned long long* fb = s_bits[tid];
+            double en = 0.0;
+            for (int e = 0; e < tk.m; ++e) {
+                const int i = ei[tk.eoff + e], j = ej[tk.eoff + e];
+                const int si = (fb[i >> 6] >> (i & 63)) & 1ull, sj = (fb[j >> 6] >> (j & 63)) & 1ull;
+                en -= (si == sj) ? ew[tk.eoff + e] : -ew[tk.eoff + e];
+            }
+            for (int i = 0; i < n; ++i) en -= ((fb[i >> 6] >> (i & 63)) & 1ull) ? -sh[i] : sh[i];
+            if (r0 + tid < restarts && en < best.e) {
+                best.e = en;
+                best.r = r0 + tid;
+                for (int w = 0; w < SA_WORDS; ++w) best.bits[w] = fb[w];
+            }
         }
-        for (int i = 0; i < n; ++i) en -= ((bits[i >> 6] >> (i & 63)) & 1ull) ? -sh[i] : sh[i];
-        if (r < restarts && en < best.e) {
-            best.e = en;
-            best.r = r;
-            for (int w = 0; w < SA_WORDS; ++w) best.bits[w] = bits[w];
-        }
-        __syncwarp();
+        __syncthreads();
     }
-    if (gl == 0) s_best[chain] = best;
+    if (tid < SA_CHAINS) s_best[tid] = best;
     __syncthreads();
     if (tid == 0) {
         int bt = 0;
@@ -292,12 +303,23 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
         if (smem > 200 * 1024) throw std::invalid_argument("instance graph too large for shared memory");
         size_t nmax = 0;
         for (const SaTask& t : tasks) nmax = std::max(nmax, (size_t)t.n);
-        smem += nmax * SA_CHAINS * sizeof(double);
         int dev = 0, sms = 0;
         SA_CK(cudaGetDevice(&dev));
         SA_CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        // Lanes per chain and kept fields.  Few chains: latency rules, 8 lanes.  From 96 chains an SM on the
+        // lanes compete, 4 of them: 296 dense n = 48, 256 restarts x 200 sweeps 24.3 ms against 28.7 with 8
+        // and 36 with 1 (64 instances: 6.5 against 6.6, 8 instances of 32 restarts: the reverse).  From 256 an
+        // SM on and at a mean degree of 8 at most, a field costs less to sum than to keep, and a chain is one
+        // thread without kept fields: 296 chains of n = 48, 96 (degree 4), 128: 9.1, 16.5, 18.8 ms against 11.9,
+        // 23.5, 30.5 with 4 lanes; dense n = 48 28.1 against 24.3.
+        const size_t chains = count * restarts;
+        const bool sum = chains >= (size_t)sms * 256 && nbr.size() <= 8 * h.size();
+        const bool fits4 = smem + nmax * (SA_THREADS / 4) * sizeof(double) <= 220 * 1024;
+        const int lanes = sum ? 1 : chains >= (size_t)sms * 96 && restarts >= 32 && fits4 ? 4 : 8;
+        const size_t per_cta = SA_THREADS / lanes;
+        if (!sum) smem += nmax * per_cta * sizeof(double);
         // CTAs per instance: one turn of restarts each, unless the batch alone fills the GPU
-        const size_t turns = (restarts + SA_CHAINS - 1) / SA_CHAINS;
+        const size_t turns = (restarts + per_cta - 1) / per_cta;
         const size_t share = std::max<size_t>(1, ((size_t)sms * SA_CTAS_PER_SM + count - 1) / count);
         const size_t ctas = std::min(turns, share);
         auto al = [](size_t x) { return (x + 255) & ~(size_t)255; };
@@ -336,10 +358,15 @@ extern "C" int tessera_qa_sa_solve(const tessera_qa_problem* problems, size_t co
         up(d_ei, ei.data(), sizeof(int) * ei.size());
         up(d_ej, ej.data(), sizeof(int) * ej.size());
         up(d_ew, ew.data(), sizeof(double) * ew.size());
-        SA_CK(cudaFuncSetAttribute(k_sa, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        k_sa<<<dim3((unsigned)count, (unsigned)ctas), SA_THREADS, smem, st>>>(d_tasks, d_off, d_nbr, d_w, d_h, d_ei, d_ej,
-                                                                          d_ew, (int)restarts, (int)sweeps, t0, t_end,
-                                                                          seed, d_part, d_tick, d_e, d_s);
+        auto run = [&](auto kern) {
+            SA_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            kern<<<dim3((unsigned)count, (unsigned)ctas), SA_THREADS, smem, st>>>(
+                d_tasks, d_off, d_nbr, d_w, d_h, d_ei, d_ej, d_ew, (int)restarts, (int)sweeps, t0, t_end, seed, d_part,
+                d_tick, d_e, d_s);
+        };
+        if (sum) run(k_sa<1, false>);
+        else if (lanes == 4) run(k_sa<4, true>);
+        else run(k_sa<8, true>);
         SA_CK(cudaGetLastError());
         std::vector<double> e(count);
         std::vector<int8_t> s(h.size());
