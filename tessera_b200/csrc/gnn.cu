@@ -87,7 +87,9 @@ __device__ __forceinline__ void ground_reduce(double best, unsigned long long bx
 // two sums' rounding bound) of the least overall and takes the reference's sum of every pattern
 // that close; its first minimum is the answer, as before.
 // Bound: a thread's set-up from the couplings, and at this size the call's own copies.  n = 22, 115
-// edges: 14 + 43 us for the two passes against 400 us for the walk over all edges.
+// edges: 14 us for the first pass; the call 79 us (98 with a chunk's second pass, 43 us, on one CTA), against
+// 400 us for the walk over all edges alone.  Where most patterns are candidates the second pass is that walk: all weights zero, whole
+// calls, n = 20: 0.20 ms (1.10 with one CTA a chunk), n = 26: 8.7 (10.2), the walk alone 8.3.
 constexpr int GS_LOW = 8;
 constexpr int GS_MIN = 16;  // patterns of one full CTA: 2^16
 constexpr int GS_NT = 256;
@@ -118,6 +120,7 @@ __global__ void __launch_bounds__(GS_NT) k_ground_scan(const double* h, const in
                             : 0.0;
     double best = INFINITY;
     unsigned long long bx = ~0ull;
+    const int l0 = (1 << GS_LOW) / gridDim.y * blockIdx.y, l1 = l0 + (1 << GS_LOW) / gridDim.y;
     for (unsigned long long c = blockIdx.x; c < chunks; c += gridDim.x) {
         if (pass && !(blk_min[c] <= cut)) continue;
         const unsigned long long hi = (c << 16) | ((unsigned long long)tid << GS_LOW);
@@ -174,7 +177,7 @@ __global__ void __launch_bounds__(GS_NT) k_ground_scan(const double* h, const in
             __syncthreads();
         } else {
 #pragma unroll 1
-            for (int l = 0; l < 1 << GS_LOW; ++l)
+            for (int l = l0; l < l1; ++l)
                 if (upper(l >> 4) + (lower(l & 15) + low[l]) <= cut) {
                     const unsigned long long x = hi | (unsigned)l;
                     const double e = ground_energy(x, h, w, ei, ej, n, m);
@@ -188,8 +191,8 @@ __global__ void __launch_bounds__(GS_NT) k_ground_scan(const double* h, const in
     if (pass) {
         ground_reduce(best, bx, re, rx);
         if (tid == 0) {
-            blk_e[blockIdx.x] = re[0];
-            blk_x[blockIdx.x] = rx[0];
+            blk_e[blockIdx.x * gridDim.y + blockIdx.y] = re[0];
+            blk_x[blockIdx.x * gridDim.y + blockIdx.y] = rx[0];
         }
     }
 }
@@ -894,7 +897,15 @@ double tessera_qa_exact_ground(const double* h, size_t n, const size_t* ei, cons
         // either sum is within (m + n + 16) roundings of `span` of the true value
         const double slack = 4.0 * (double)(m + n + 16) * 2.3e-16 * span;
         const unsigned long long chunks = scan ? 1ull << (n - 16) : 0;
-        if (scan) blocks = std::min<unsigned long long>(chunks, (unsigned long long)nsm * 2);
+        // the second pass splits a chunk's patterns over `parts` CTAs: in degenerate instances it sums
+        // nearly every pattern
+        unsigned long long grid = 0;
+        unsigned parts = 1;
+        if (scan) {
+            grid = std::min<unsigned long long>(chunks, (unsigned long long)nsm * 2);
+            while (parts < 8 && grid * parts * 2 <= (unsigned long long)nsm * 8) parts *= 2;
+            blocks = grid * parts;
+        }
         auto al = [](size_t sz) { return (sz + 63) & ~(size_t)63; };
         // one upload: h, w, ei, ej (and the least sum's start); one download: every CTA's energy
         // and pattern
@@ -932,7 +943,7 @@ double tessera_qa_exact_ground(const double* h, size_t n, const size_t* ei, cons
         if (err == cudaSuccess) {
             if (scan) {
                 for (int pass = 0; pass < 2; ++pass)
-                    k_ground_scan<<<(unsigned)blocks, GS_NT>>>(dh, di, dj, dw, (double*)(arena + o_d), loops, (int)n,
+                    k_ground_scan<<<dim3((unsigned)grid, pass ? parts : 1), GS_NT>>>(dh, di, dj, dw, (double*)(arena + o_d), loops, (int)n,
                                                                (int)m, pass, slack, bm, dl, be, bx);
             } else {
                 k_ground<<<(unsigned)blocks, 256, smem>>>(dh, di, dj, dw, (int)n, (int)m, total, be, bx);
