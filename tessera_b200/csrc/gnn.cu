@@ -468,26 +468,28 @@ __global__ void k_node_head_bwd(Wt W, size_t own, const float* p, const float* t
 // weight gradient of a linear map: dW[o][k] += sum_r d[r][o] in(r, k), db[o] += sum_r d[r][o], where
 // input row r = [in0[idx0 ? idx0[r] : r][0..K0), in1[r][0..K1), in2[r] (if in2)]
 // With msk, d[r][o] stands for d[dix[r]][o] where msk[r][o] > 0 and 0 elsewhere (the message
-// gradient, not formed on its own).  Each CTA takes one output tile over WG_ROWS rows and adds it to
-// the gradient.  One thread per weight walked all rows before: 348 us a launch at 320 nodes and 1600
+// gradient, not formed on its own).  Each CTA takes one output tile over WG_ROWS rows at a time and adds
+// it to the gradient.  One thread per weight walked all rows before: 348 us a launch at 320 nodes and 1600
 // edges, 2.8 of a training step's 3.1 ms.
 constexpr int WG_ROWS = 128;
 __global__ void __launch_bounds__(GT_NT) k_wgrad_lin(const float* d, const int* dix, const float* msk, int rows,
                                                      int H_out, const float* in0, const int* idx0, int K0,
                                                      const float* in1, int K1, const float* in2, float* gW, float* gb) {
     const int Kt = K0 + K1 + (in2 ? 1 : 0);
-    const int q0 = blockIdx.z * WG_ROWS, q1 = q0 + WG_ROWS < rows ? q0 + WG_ROWS : rows;
-    gemm_tile(blockIdx.x * GT, blockIdx.y * GT, H_out, Kt + 1, q0, q1,
-              [&](int o, int r) {
-                  if (msk) return msk[(size_t)r * H_out + o] > 0.f ? d[(size_t)dix[r] * H_out + o] : 0.f;
-                  return d[(size_t)r * H_out + o];
-              },
-              [&](int r, int k) {
-                  if (k < K0) return in0[(size_t)(idx0 ? idx0[r] : r) * K0 + k];
-                  if (k < K0 + K1) return in1[(size_t)r * K1 + (k - K0)];
-                  return k < Kt ? in2[r] : 1.f;
-              },
-              [&](int o, int k, float v) { atomicAdd(k < Kt ? &gW[(size_t)o * Kt + k] : &gb[o], v); });
+    for (long long q = (long long)blockIdx.z * WG_ROWS; q < rows; q += (long long)gridDim.z * WG_ROWS) {
+        const int q0 = (int)q, q1 = (int)(q + WG_ROWS < rows ? q + WG_ROWS : rows);
+        gemm_tile(blockIdx.x * GT, blockIdx.y * GT, H_out, Kt + 1, q0, q1,
+                  [&](int o, int r) {
+                      if (msk) return msk[(size_t)r * H_out + o] > 0.f ? d[(size_t)dix[r] * H_out + o] : 0.f;
+                      return d[(size_t)r * H_out + o];
+                  },
+                  [&](int r, int k) {
+                      if (k < K0) return in0[(size_t)(idx0 ? idx0[r] : r) * K0 + k];
+                      if (k < K0 + K1) return in1[(size_t)r * K1 + (k - K0)];
+                      return k < Kt ? in2[r] : 1.f;
+                  },
+                  [&](int o, int k, float v) { atomicAdd(k < Kt ? &gW[(size_t)o * Kt + k] : &gb[o], v); });
+    }
 }
 
 __global__ void k_relu_mask(const float* g, const float* pre, int n, float* out) {
@@ -668,7 +670,7 @@ public:
     void wgrad(const float* d, const int* dix, const float* msk, int rows, int H_out, const float* in0, const int* idx0,
                int K0, const float* in1, int K1, const float* in2, float* gW, float* gb) {
         dim3 grid = tiles(H_out, K0 + K1 + (in2 ? 1 : 0) + 1);
-        grid.z = (rows + WG_ROWS - 1) / WG_ROWS;
+        grid.z = std::min((rows + WG_ROWS - 1) / WG_ROWS, 65535);  // the most a grid's third dimension takes
         k_wgrad_lin<<<grid, GT_NT, 0, st>>>(d, dix, msk, rows, H_out, in0, idx0, K0, in1, K1, in2, gW, gb);
     }
 
