@@ -57,9 +57,11 @@ static int g_fail_after = 0, g_fail_count = 0;
 // plain memory, as it is made once.  The pool holds at most kKeep bytes per device, grows by kGrow at a
 // time (a growth of a few MB per allocation made 100 small engines take 1 ms each), and an allocation
 // that would take it beyond kKeep is a plain cudaMalloc.  What the pool holds unused goes back to the
-// driver when an allocation fails or device_trim() is called, and the pools end with the process.  Allocation and release run on a stream of the pool's own that no
-// kernel uses, and are waited for, so the memory is good for any stream and thread when alloc()
-// returns; callers have waited for their work before they free, as cudaFree's callers had not to.
+// driver when an allocation fails or device_trim() is called, and the pools end with the process.
+// Allocation and release run on a stream of the pool's own that no kernel uses, and are waited for, so the
+// memory is good for any stream and thread when alloc() returns; callers have waited for their work before
+// they free, as cudaFree's callers had not to.  A lock per device: threads on different GPUs, and those
+// that only take plain memory, do not wait for one another.
 class DevicePools {
 public:
     static DevicePools& get() {
@@ -70,46 +72,43 @@ public:
         int dev = 0;
         cudaError_t e = cudaGetDevice(&dev);
         if (e != cudaSuccess) return e;
-        std::lock_guard<std::mutex> lk(mu_);
-        Pool* pl = pool(dev);
-        const bool pooled = want && pl && pl->used + bytes <= kKeep;
-        if (pooled) grow(*pl, bytes);
-        for (int turn = 0; turn < 2; ++turn) {
-            if (pooled) {
-                e = cudaMallocFromPoolAsync(out, bytes, pl->pool, pl->st);
-                if (e == cudaSuccess) e = cudaStreamSynchronize(pl->st);
-            } else {
-                e = cudaMalloc(out, bytes);
-            }
-            if (e != cudaErrorMemoryAllocation || !pl) break;
-            cudaGetLastError();  // not sticky: the caller reports it, or the second turn succeeds
-            if (turn == 0) cudaMemPoolTrimTo(pl->pool, 0);
-        }
-        if (e == cudaSuccess && pooled) {
-            owner_[*out] = Block{dev, bytes};
-            pl->used += bytes;
-        }
+        Pool* pl = dev >= 0 && dev < kMax ? &pools_[dev] : nullptr;
+        if (want && pl && from_pool(out, bytes, dev, *pl, e)) return e;
+        e = cudaMalloc(out, bytes);
+        if (e != cudaErrorMemoryAllocation) return e;
+        cudaGetLastError();  // not sticky: the caller reports it, or the second turn succeeds
+        trim();
+        e = cudaMalloc(out, bytes);
+        if (e == cudaErrorMemoryAllocation) cudaGetLastError();
         return e;
     }
     void free(void* p) {
         if (!p) return;
-        std::unique_lock<std::mutex> lk(mu_);
-        auto it = owner_.find(p);
-        if (it == owner_.end()) {
-            lk.unlock();
+        Block b;
+        {
+            std::lock_guard<std::mutex> lk(owner_mu_);
+            auto it = owner_.find(p);
+            if (it == owner_.end()) b.dev = -1;
+            else {
+                b = it->second;
+                owner_.erase(it);
+            }
+        }
+        if (b.dev < 0) {
             cudaFree(p);
             return;
         }
-        Pool& pl = pools_[it->second.dev];
-        pl.used -= it->second.bytes;
-        owner_.erase(it);
+        Pool& pl = pools_[b.dev];
+        std::lock_guard<std::mutex> lk(pl.mu);
+        pl.used -= b.bytes;
         cudaFreeAsync(p, pl.st);
         cudaStreamSynchronize(pl.st);
     }
     void trim() {
-        std::lock_guard<std::mutex> lk(mu_);
         int dev = 0;
-        if (cudaGetDevice(&dev) == cudaSuccess && dev < kMax && pools_[dev].state == 1) cudaMemPoolTrimTo(pools_[dev].pool, 0);
+        if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMax) return;
+        std::lock_guard<std::mutex> lk(pools_[dev].mu);
+        if (pools_[dev].state == 1) cudaMemPoolTrimTo(pools_[dev].pool, 0);
     }
 
 private:
@@ -117,6 +116,7 @@ private:
     static constexpr uint64_t kKeep = 256ull << 20;
     static constexpr uint64_t kGrow = 64ull << 20;
     struct Pool {
+        std::mutex mu;  // of this device alone, and not held across plain allocations
         int state = 0;  // 0 not tried, 1 ready, 2 not to be had on this device
         cudaMemPool_t pool = nullptr;
         cudaStream_t st = nullptr;
@@ -126,6 +126,24 @@ private:
         int dev;
         size_t bytes;
     };
+    // whether the pool of the current device had the memory; e: what went wrong otherwise
+    bool from_pool(void** out, size_t bytes, int dev, Pool& pl, cudaError_t& e) {
+        std::lock_guard<std::mutex> lk(pl.mu);
+        if (!ready(dev, pl) || pl.used + bytes > kKeep) return false;
+        grow(pl, bytes);
+        for (int turn = 0; turn < 2; ++turn) {
+            e = cudaMallocFromPoolAsync(out, bytes, pl.pool, pl.st);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(pl.st);
+            if (e != cudaErrorMemoryAllocation) break;
+            cudaGetLastError();
+            if (turn == 0) cudaMemPoolTrimTo(pl.pool, 0);
+        }
+        if (e != cudaSuccess) return true;
+        pl.used += bytes;
+        std::lock_guard<std::mutex> ok(owner_mu_);
+        owner_[*out] = Block{dev, bytes};
+        return true;
+    }
     // takes and returns a block of kGrow when the next allocation would make the pool grow
     void grow(Pool& pl, size_t bytes) {
         uint64_t held = 0;
@@ -136,9 +154,7 @@ private:
         if (cudaMallocFromPoolAsync(&p, kGrow, pl.pool, pl.st) == cudaSuccess) cudaFreeAsync(p, pl.st);
         else cudaGetLastError();
     }
-    Pool* pool(int dev) {  // dev is current; nullptr: plain cudaMalloc
-        if (dev < 0 || dev >= kMax) return nullptr;
-        Pool& pl = pools_[dev];
+    bool ready(int dev, Pool& pl) {  // dev is current
         if (pl.state == 0) {
             pl.state = 2;
             int ok = 0;
@@ -156,10 +172,10 @@ private:
             else
                 cudaGetLastError();
         }
-        return pl.state == 1 ? &pl : nullptr;
+        return pl.state == 1;
     }
-    std::mutex mu_;
     Pool pools_[kMax];
+    std::mutex owner_mu_;
     std::unordered_map<void*, Block> owner_;
 };
 
