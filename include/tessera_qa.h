@@ -86,8 +86,8 @@ typedef struct tessera_qa_config {
     double jacobi_tol;      /* rotate a column pair when |w_p^H w_q| > tol |w_p||w_q|; 0 = default */
     int jacobi_max_sweeps;  /* 0 = default (60) */
     int jacobi_block;       /* 0 = chosen by size (resident Jacobi for small theta, else column pairs in blocks
-                               of 8); 1,2,4,8,16 = column-pair blocks of that width; 32 = block-Gram Jacobi
-                               (batches) */
+                               of 8, 4 or 16); 1,2,4,8,16 = column-pair blocks of that width (batches: at least
+                               4, and 16 only up to 256 rows in complex128); 32 = block-Gram Jacobi (batches) */
     int device;             /* CUDA device ordinal; -1 = the calling thread's current device */
     size_t step_begin;      /* run schedule steps [step_begin, step_end) */
     size_t step_end;        /* 0 = problem.steps */

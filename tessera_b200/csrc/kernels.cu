@@ -3583,16 +3583,14 @@ static void svd_batch_bw(const InstTask<T>* insts, const UpdRef* refs, int nref,
     TQ_CHECK(cudaGetLastError());
 }
 
-// complex64: blocks of 16 columns (512 threads, 16 warps); complex128 columns do not fit in the
-// registers that 16 warps leave each thread
-template <typename T, int RPL>
-static bool svd_batch_wide(int bw, int rpl, const InstTask<T>* insts, const UpdRef* refs, int nref, int rows_cap,
-                           cudaStream_t s, int lq) {
+// complex64 at 512 rows: blocks of 16 columns (512 threads, 16 warps); complex128 columns of 512 rows do
+// not fit in the registers that 16 warps leave each thread
+template <typename T>
+static bool svd_batch_wide(const InstTask<T>* insts, const UpdRef* refs, int nref, int rows_cap, cudaStream_t s,
+                           int lq) {
     if constexpr (sizeof(T) == 4) {
-        if (bw == 16 && rpl == RPL) {
-            svd_batch_bw<T, 16, RPL>(insts, refs, nref, rows_cap, s, lq);
-            return true;
-        }
+        svd_batch_bw<T, 16, 16>(insts, refs, nref, rows_cap, s, lq);
+        return true;
     }
     return false;
 }
@@ -3628,7 +3626,6 @@ int launch_update_batch(const InstTask<T>* insts, const UpdRef* refs, int nref, 
     // one asked for; complex64 at 257..512 rows: 16), or the block-Gram kernel when block width
     // 32 is asked for
     if (block_w == 0) bw = (sizeof(T) == 4 && rpl == 16) ? 16 : 8;
-    if (sizeof(T) == 8 && bw > 8) bw = 8;  // two columns a warp: 16 warps leave too few registers
     // the pivoted LQ preconditioner for the column-pair kernel (outside the svd_begin/svd_end window,
     // so that window times the Jacobi alone): complex64 at 257..512 rows, complex128 wherever theta
     // is not resident
@@ -3644,14 +3641,14 @@ int launch_update_batch(const InstTask<T>* insts, const UpdRef* refs, int nref, 
     if (res_dispatch<T>(nullptr, nullptr, rp, insts, refs, nref, s)) {
     } else if (block_w == BG_B) {
         bgj_launch<T>(nullptr, nullptr, nullptr, insts, refs, nref, s);
-    } else if (svd_batch_wide<T, 16>(bw, rpl, insts, refs, nref, rows_cap, s, lq)) {
+    } else if (bw == 16 && rpl == 16 && svd_batch_wide<T>(insts, refs, nref, rows_cap, s, lq)) {
     } else {
 #define TQ_RB(B, RP) \
     if (bw == B && rpl == RP) { svd_batch_bw<T, B, RP>(insts, refs, nref, rows_cap, s, lq); } else
         // (theta up to 64 rows is resident in either precision)
         TQ_RB(4, 4) TQ_RB(4, 8) TQ_RB(4, 16) TQ_RB(8, 4) TQ_RB(8, 8) TQ_RB(8, 16)
-        if (!svd_batch_wide<T, 8>(bw, rpl, insts, refs, nref, rows_cap, s, lq))
-            throw std::runtime_error("unsupported Jacobi block width");
+        TQ_RB(16, 4) TQ_RB(16, 8)
+        throw std::runtime_error("unsupported Jacobi block width");
 #undef TQ_RB
     }
     if (svd_end) TQ_CHECK(cudaEventRecord(svd_end, s));
