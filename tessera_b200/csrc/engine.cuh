@@ -96,6 +96,10 @@ struct SvdParams {
                        //    rank-revealing LQ before its Jacobi
 };
 
+// complex128 theta this small go to their batched Jacobi as they are in a launch whose bounds called for the
+// LQ (an anneal's first steps: bonds of a few columns under a large cap)
+__host__ __device__ inline bool lq_skips(int R, int N) { return R <= 8 && N <= 8; }
+
 struct ChainStep {
     int site;
     int zflag;

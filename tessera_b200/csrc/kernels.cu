@@ -2455,7 +2455,7 @@ __device__ void svd_body_rcd(const MpsView<double>& mps, const SvdWork<double>& 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int R = pp.R > 0 ? pp.R : 2 * mps.dims[pp.bond];
     const int N0 = pp.N > 0 ? pp.N : 2 * mps.dims[pp.bond + 2];
-    const int N = pp.lq && N0 > R ? R : N0;
+    const int N = pp.lq && N0 > R && !lq_skips(R, N0) ? R : N0;
     constexpr int rc = 32 * RPL;  // staged column length; the rows from R on stay zero
     const int ld = wk.ld;
     double2* W = wk.W;

@@ -493,6 +493,7 @@ __global__ void __launch_bounds__(LQ_NT, 1) k_lq_batch(const InstTask<T>* insts,
         const UpdRef rf = refs[t];
         const InstTask<T>& it = insts[rf.inst];
         const int R = 2 * it.mps.dims[rf.op.bond], N = 2 * it.mps.dims[rf.op.bond + 2];
+        if (sizeof(T) == 8 && lq_skips(R, N)) continue;
         if constexpr (sizeof(T) == 8) lq_block_body(it.wk.W, it.wk.ld, R, N, &it.wk.stats->status, smraw);
         else lq_body<T>(it.wk.W, it.wk.ld, R, N, &it.wk.stats->status, smraw);
         __syncthreads();
