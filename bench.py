@@ -278,6 +278,25 @@ class RefModel:
                        f"chi={self.chi // 2} ({self.t_lo:.2f} s) and chi={self.chi} at the same concurrency")
 
 
+TRAFFIC = os.path.join(ROOT, "profiles", "k_svd_traffic.json")
+
+
+def captured_traffic(args, batch, counted):
+    """DRAM bytes of one Jacobi launch as a profiler captured them, if the capture is of this workload and of
+    this kernel: `counted`, the bytes a launch of this run counted itself, is within 15% of what the captured
+    one counted (sweeps differ a little between windows; another kernel's traffic differs by more)."""
+    try:
+        with open(TRAFFIC) as f:
+            d = json.load(f)
+        same = (d["chi"] == args.chi and d["precision"] == args.precision and d["batch"] == batch
+                and d["jacobi_precondition"] == args.precondition)
+        if same and abs(counted / d["counted_bytes_per_launch"] - 1.0) < 0.15:
+            return d["dram_bytes_per_launch"]
+    except (OSError, ValueError, KeyError):
+        pass
+    return None
+
+
 def run_reference(args):
     rank = int(os.environ.get("RANK", "0"))
     if rank != 0:
@@ -549,7 +568,8 @@ def main():
     if args.profile_run:
         step(0)
         r = sess.sync()
-        print(f"profile run: {r.two_site_updates} updates, status {r.status}, {r.device_ms:.1f} ms")
+        print(f"profile run: {r.two_site_updates} updates, status {r.status}, {r.device_ms:.1f} ms, "
+              f"{r.svd_bytes:.4g} bytes counted by {r.svd_launches} Jacobi launches")
         return
     for w in range(args.warmup):
         step(w)
@@ -588,17 +608,7 @@ def main():
     sweeps = (r1.svd_sweeps - r0.svd_sweeps) / max(updates, 1)
     peak, peak_kind = peaks()
     achieved = (svd_bytes / svd_n) / (svd_ms / svd_n / 1e3) / 1e9 if svd_n else 0.0
-    traffic = None
-    tf = os.path.join(ROOT, "profiles", "k_svd_traffic.json")
-    if os.path.exists(tf):
-        try:
-            with open(tf) as f:
-                d = json.load(f)
-            if (d.get("chi") == args.chi and d.get("precision") == args.precision and d.get("batch") == B
-                    and d.get("jacobi_precondition", "off") == args.precondition):
-                traffic = d.get("dram_bytes_per_launch")
-        except Exception:
-            traffic = None
+    traffic = captured_traffic(args, B, svd_bytes / svd_n if svd_n else 0.0)
     if B == 1:
         kname = "k_svd (cooperative column-pair Jacobi, 512x512 theta)"
     elif args.jacobi_block == 32:
