@@ -649,7 +649,7 @@ __device__ __forceinline__ int pair_tracked(double2* col, const int rc, const in
 // per block); the whole grid meets only at the end of a sweep.  Changed columns go back by bulk
 // copies.  complex128 carries norms and takes angles as svd_body_rcd does.  512 x 512 complex128
 // after the LQ, 11 sweeps: 12.6 ms with a grid barrier a round, 32 CTAs and element-wise stores,
-// 11.2 ms now; complex64 400 x 400: 7.3 -> 5.9 ms.  Bound: a round's chain on 64 of 148 SMs (stage
+// 11.4 ms now (12.2 where it takes 12); complex64 400 x 400: 7.3 -> 5.9 ms.  Bound: a round's chain on 64 of 148 SMs (stage
 // 64 KB, four dependent visits, store, flag); the pair arithmetic alone made no difference (13.5 ms
 // with 32 CTAs and the barrier).
 template <typename T, int BW, int RPL>
@@ -1135,7 +1135,7 @@ __device__ int lq_resident(double2* col, const int rc, const int R, const int N,
             left += __shfl_xor_sync(0xffffffffu, left, o);
             if (b2 > best || (b2 == best && p2 < p)) { best = b2; p = p2; }
         }
-        if (left != left) return N;  // not a number: every column stays in, and raises the status
+        if (left != left) return N;  // not a number: every column stays in
         if (!(left > 1e-6 * tiny) || !(best > 0.0)) break;
         // reflector u = (e (|x_0| + alpha), x_1, ...) of that row's columns >= k
         const double2 x0 = col[k * rc + p];

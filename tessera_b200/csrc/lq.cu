@@ -701,7 +701,7 @@ __global__ void __launch_bounds__(LQC_NT, 1) k_lq_coop(MpsView<T> mps, int bond,
 // per sixteen steps instead of sixteen.  The buffers need no second copy: norms are read before the
 // second barrier and written after it, panel rows read before the next panel's first and written
 // after it.  Barrier timeouts leave theta in W, as in k_lq_coop.  512 x 512: 3.9 -> 2.8
-// ms (the Jacobi after it 11.2 -> 11.9 ms, 12 sweeps instead of 11 on one theta); 200 x 200: 1.4 -> 0.9
+// ms (the Jacobi after it takes 11 or 12 sweeps, 11.4 or 12.2 ms, where it took 11); 200 x 200: 1.4 -> 0.9
 // ms.  Bound: the panel's sixteen steps, which every CTA takes in turn.
 // ------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(LQ_NT, 1) k_lq_coop_block(MpsView<double> mps, int bond, SvdWork<double> wk,
