@@ -740,7 +740,7 @@ public:
         TQ_CK(cudaMemcpyAsync(da, a, sizeof(V) * (size_t)R * N, cudaMemcpyHostToDevice, stream_));
         launch_svd_load<T>(da, R, N, W_, ld_, stream_);
         const int bw = pick_block(R, N);
-        launch_svd<T>(mps(), 0, k, tol_for(R, false), C_.max_sweeps, work(), R, N, bw, stream_, R, N);
+        launch_svd<T>(mps(), 0, k, tol_for(R, true), C_.max_sweeps, work(), R, N, bw, stream_, R, N);
         if (u || vh) launch_svd_u<T>(W_, ld_, perm_, sig_, R, k, du, stream_);
         std::vector<double> sg(k);
         RunStats st;
@@ -876,6 +876,8 @@ private:
     // drifts with them: over 660 updates of n = 12, chi = 64 by 7.9e-12 (rms) at 1e-13 against 6.2e-12 without
     // the LQ, by 1.5e-12 at 2e-14, for under 2% of time (9.0 sweeps instead of 8.9).  A batch above 256 rows,
     // which has always had the LQ, stays at 1e-13 (2e-14 would cost it 9.8 sweeps instead of 9.4).
+    // The standalone SVD is fine too: its factors are what leftovers reach first (320 x 320: isometry of vh
+    // 5.8e-11 -> 0.95e-11, 8.55 -> 8.66 ms a call; of u 1e-13 -> 2e-14).
     double tol_for(int R, bool fine) const {
         if (C_.tol > 0) return C_.tol;
         const double eps = sizeof(T) == 8 ? 2.220446049250313e-16 : 1.1920928955078125e-07;
